@@ -41,8 +41,10 @@ enum {
 
 /* precision of the per-pixel path */
 enum {
-  P2M_PREC_FP64 = 0,  /* plain drop-in: FP64 pixel geometry (pix2vec_ring + angdist) for
-                         every candidate, FP64 accumulation */
+  P2M_PREC_FP64 = 0,  /* plain drop-in: the result of FP64 pixel geometry (pix2vec_ring +
+                         angdist) for every candidate, FP64 accumulation.  A candidate whose
+                         float angle a float-float computation already settles skips the
+                         double-precision arithmetic; the others go through it */
   P2M_PREC_MIXED = 1, /* FP32 disc test and profile interpolation with an exact FP64
                          recheck near every decision boundary; compensated FP32
                          accumulation: the float maps hold the high words, the exact
@@ -65,8 +67,9 @@ enum {
                                P2M_SET_CAP read by p2m_create; more is P2M_ERR_CAPACITY */
   P2M_FLAG_ALL_HALOS = 2,   /* enumerate halos whose table value is identically zero */
   P2M_FLAG_TIMING = 4,      /* record per-phase device times (p2m_get_timings) */
-  P2M_FLAG_VALIDATE = 8     /* mixed precision: also run the exact path for every candidate
-                               and count disagreements (p2m_stats.val_*); slow */
+  P2M_FLAG_VALIDATE = 8     /* also run the exact path for every candidate and count
+                               disagreements (p2m_stats.val_*; with P2M_PREC_FP64 of the
+                               table index or the bits of its fraction); slow */
 };
 
 #define P2M_MAXMAPS 8

@@ -40,7 +40,7 @@ struct p2m_ctx {
   unsigned int *d_fits[2] = {nullptr, nullptr}, *h_fits[2] = {nullptr, nullptr};
   cudaEvent_t ev_fits[2] = {nullptr, nullptr};
   float4 *d_ringtab = nullptr;
-  float2 *d_ringhd = nullptr;
+  float4 *d_ringaux = nullptr;
   float4 *d_phitab = nullptr;
   /* scramble / centre of the catalogue (pks2map.f90:162-262) */
   p2m_pre pre = {};
@@ -242,7 +242,7 @@ PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
   P.rofz = ctx->d_rofz;
   P.zofr = ctx->d_zofr;
   P.ringtab = ctx->d_ringtab;
-  P.ringhd = ctx->d_ringhd;
+  P.ringaux = ctx->d_ringaux;
   P.phitab = ctx->d_phitab;
   P.pre = ctx->pre;
   P.pre_ord = ctx->d_pre_ord;
@@ -256,12 +256,20 @@ PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
   P.halos_threads = ctx->tune.halos_threads;
   P.err_flag = &ctx->d_ctr->err;
   P.cone_npix = ctx->cone_npix;
+  P.neg_zero = -0.0f;
   if (ctx->th_set) {
     float fr;
     int ir;
     p2m_rindex(&ctx->th, FMUL(ctx->th.rmint, 0.5f), &ir, &fr);
     P.ir_c = ir;
     P.fr_c = fr;
+    const float dr = 1e-5f;
+    P.r_out = ctx->th.rmaxt * (1.0f + dr);
+    P.r_in = ctx->th.rmaxt * (1.0f - dr);
+    P.r_min_in = ctx->th.rmint * (1.0f + dr);
+    P.r_min_out = ctx->th.rmint * (1.0f - dr);
+    P.row_m = ctx->th.nrt;
+    P.row_c = ctx->th.nrt * ctx->th.nmht;
   }
   return P;
 }
@@ -757,10 +765,8 @@ p2m_status p2m_create(const p2m_config *cfg, p2m_ctx **out) {
   ctx->cfg = *cfg;
   *out = ctx;
   if (const char *e = getenv("P2M_BAND_U")) ctx->band_u = (float)atof(e);
-  /* the plain FP64 path is fastest with every halo on the stored-item path, which balances
-     its heavy per-candidate work over candidates; test hook: P2M_BIG_RINGS routes every
-     halo through one painting path (0: stored items only) */
-  if (cfg->precision == P2M_PREC_FP64) ctx->tune.big_rings = 0;
+  /* test hook: P2M_BIG_RINGS routes every halo through one painting path (0: stored items
+     only) */
   if (const char *e = getenv("P2M_BIG_RINGS")) ctx->tune.big_rings = std::max(0, atoi(e));
   CK(cudaSetDevice(cfg->device));
   CK(cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, cfg->device));
@@ -791,19 +797,24 @@ p2m_status p2m_create(const p2m_config *cfg, p2m_ctx **out) {
     }
     CK(cudaMalloc((void **)&ctx->d_ringtab, sizeof(float4) * (size_t)nr));
     CK(cudaMemcpy(ctx->d_ringtab, rt.data(), sizeof(float4) * (size_t)nr, cudaMemcpyHostToDevice));
-    /* pi / npr of each ring as a (hi, lo) float pair: the candidates' longitude step */
-    std::vector<float2> hd((size_t)nr);
-    hd[0] = make_float2(0.0f, 0.0f);
+    /* pi / npr of each ring as a (hi, lo) float pair (the candidates' longitude step), its
+       first pixel, and its pixel count with the longitude shift */
+    std::vector<float4> aux((size_t)nr);
+    aux[0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int r = 1; r < nr; r++) {
       int npr, ks;
       long long npn;
       p2m_ring_info(cfg->nside, r, &npr, &ks, &npn);
       const double v = P2M_HP_PI / (double)npr;
       const float vh = (float)v;
-      hd[(size_t)r] = make_float2(vh, (float)(v - (double)vh));
+      const int first = (int)(npn - npr), info = 2 * npr + ks; /* npix <= 12 * 8192^2 < 2^31 */
+      float4 a = make_float4(vh, (float)(v - (double)vh), 0.0f, 0.0f);
+      memcpy(&a.z, &first, 4);
+      memcpy(&a.w, &info, 4);
+      aux[(size_t)r] = a;
     }
-    CK(cudaMalloc((void **)&ctx->d_ringhd, sizeof(float2) * (size_t)nr));
-    CK(cudaMemcpy(ctx->d_ringhd, hd.data(), sizeof(float2) * (size_t)nr, cudaMemcpyHostToDevice));
+    CK(cudaMalloc((void **)&ctx->d_ringaux, sizeof(float4) * (size_t)nr));
+    CK(cudaMemcpy(ctx->d_ringaux, aux.data(), sizeof(float4) * (size_t)nr, cudaMemcpyHostToDevice));
     /* cos and sin of the grid angles 2 pi k / M as (hi, lo) float pairs */
     std::vector<float4> pt(P2M_PHITAB);
     for (int k = 0; k < P2M_PHITAB; k++) {
@@ -869,7 +880,7 @@ void p2m_destroy(p2m_ctx *ctx) {
   cudaSetDevice(ctx->cfg.device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->zstream) cudaStreamSynchronize(ctx->zstream);
-  void *ptrs[] = {ctx->d_rofz, ctx->d_zofr, ctx->d_ringtab, ctx->d_ringhd, ctx->d_phitab, ctx->d_acc64, ctx->d_fs_acc,
+  void *ptrs[] = {ctx->d_rofz, ctx->d_zofr, ctx->d_ringtab, ctx->d_ringaux, ctx->d_phitab, ctx->d_acc64, ctx->d_fs_acc,
                   ctx->d_fs_out, ctx->d_halos, ctx->d_items_raw,
                   ctx->d_nring, ctx->d_ioff, ctx->d_fs_items, ctx->d_scan_tmp, ctx->d_counts,
                   ctx->d_pix_off, ctx->d_nitems, ctx->d_sums, ctx->d_set_rec, ctx->d_set_pix,

@@ -164,11 +164,16 @@ P2M_HD float p2m_logf(float x) {
   return FADD(FMUL(fe, P2M_LN2_HI), FADD(lm, FMUL(fe, P2M_LN2_LO)));
 }
 
-/* p2m_logf for a positive, normal, finite x, without the special-value tests (which
-   such an x never takes): the same result bit for bit */
+/* p2m_logf for a positive, normal, finite x, without the special-value and subnormal
+   tests (which such an x never takes): the same result bit for bit */
 P2M_HD float p2m_logf_normal(float x) {
-  int e;
-  float m = p2m_frexp_centered(x, &e);
+  uint32_t u = p2m_f2u(x);
+  int e = (int)(u >> 23) - 127;
+  float m = p2m_u2f((u & 0x007fffffu) | 0x3f800000u);
+  if (m > P2M_SQRT2) {
+    m = FMUL(m, 0.5f);
+    e += 1;
+  }
   float lm = p2m_log_core(m);
   float fe = (float)e;
   return FADD(FMUL(fe, P2M_LN2_HI), FADD(lm, FMUL(fe, P2M_LN2_LO)));

@@ -59,32 +59,33 @@ struct HaloRec {
   float T;                /* dtheta_halo (float value), haloproject.f90:47 */
   float C_in, C_out, C_span; /* chord^2 thresholds: certainly inside / outside / span */
   float chi_t, fc, fm;    /* per-halo part of interpolate_table */
-  int ichi, imh, zero;
+  int ichi, imh;
+  int zc;                 /* bit 0: the table value is identically zero; bits 1..: light-cone of
+                             an ensemble (the maps' slot offset is cone * 12 nside^2) */
   float w1, w2;           /* deposit weights of profile-1 and profile-2 maps */
-  int cone;               /* light-cone of an ensemble: the maps' slot offset is
-                             cone * 12 nside^2 (0 outside ensembles) */
+  int cb;                 /* float2 index of table row (imh, ichi) at ir = 1 when the rows of
+                             all four corners lie inside the table; -1: clamped offsets */
   long long rec;          /* record index (over all paint calls since the reset) */
   int ir_lo, ir_hi;       /* candidate rings */
-  int cbase[4];           /* table offsets of corners (imh,ichi),(imh+1,ichi),(imh,ichi+1),
-                             (imh+1,ichi+1) at ir=1, profile 1; -1: clamped offsets */
   float theta_h, phi_h;   /* flat-sky centre (float values), haloproject.f90:105-106 */
   int jmin, jmax, kmin, kmax; /* flat-sky box; jmin > jmax: none */
 };
+/* one 128-byte line per halo: every reader and writer of a record touches one line */
+static_assert(sizeof(HaloRec) == 128, "HaloRec layout");
 
 /* candidate span of one ring of one disc */
-static_assert(sizeof(HaloRec) == 144, "HaloRec layout");
 
 struct RingItem {
   int halo;
   int ring_n0;               /* ring << 16 | (n0 & 0xffff) */
   int lo, count;             /* lo: unwrapped phi index of the first candidate */
-  float A, B;                /* chord^2 = A + B sin^2(dphi/2) */
-  float f0;                  /* x0 = (lo + kshift/2) - phi0 npr / 2pi = n0 + f0 (pixel units):
-                                the k-th candidate sits at x = (n0 + k) + f0, exact integer
-                                part, so x keeps full relative precision near the centre */
-  float hdphi;               /* pi / npr */
-  float Al, Bl, f0l, hdl;    /* low words: (A, Al), (B, Bl), (f0, f0l), (hdphi, hdl) are
-                                float-float values (~44 bits) for the pixel's angle */
+  /* float-float (hi, lo) values (~44 bits) of the pixel's angle.  chord^2 = A + B sin^2(y)
+     with y half the longitude offset from the disc centre.  The first candidate sits at
+     (lo + kshift/2) - phi0 npr / 2pi = n0 + f0 pixels; the k-th has y = (n0 + k) d + y0
+     with d = pi / npr and y0 = f0 d: the integer part is exact, so y keeps full relative
+     precision near the centre */
+  float4 ab;                 /* A hi, A lo, B hi, B lo */
+  float4 yd;                 /* y0 hi, y0 lo, d hi, d lo */
 };
 static_assert(sizeof(RingItem) == 48, "RingItem layout");
 
@@ -109,6 +110,10 @@ struct PaintParams {
   float fr_c;
   float band_u;  /* half-width of the r-index recheck band (cell units) */
   float inv_drt; /* 1 / drt of the table */
+  float r_out, r_in, r_min_in, r_min_out; /* rmaxt (1 +- 1e-5) and rmint (1 -+ 1e-5): radii
+                    between a pair are left to the exact path */
+  float neg_zero;   /* -0: see mul2_sep */
+  int row_m, row_c; /* float2 entries from a table row to the next mass and the next chi */
   int big_rings; /* halos spanning more rings are painted from stored items */
   const float *tables[P2M_MAXTABLES];
   /* maps 2q and 2q + 1 as one table of float2 entries (.x map 2q, .y map 2q + 1) at the
@@ -117,7 +122,8 @@ struct PaintParams {
   const float2 *pair_tab[P2M_MAXMAPS / 2];
   const float *rofz, *zofr;
   const float4 *ringtab; /* (z hi, z lo, sin theta hi, sin theta lo) of ring i at index i */
-  const float2 *ringhd;  /* pi / npr of ring i as (hi, lo) */
+  const float4 *ringaux; /* ring i: pi / npr as (hi, lo), then as ints the RING index of its
+                            first pixel and 2 npr + kshift */
   const float4 *phitab;  /* (cos hi, cos lo, sin hi, sin lo) of 2 pi k / P2M_PHITAB */
   p2m_pre pre;           /* scramble / centre of the catalogue (pks2map.f90:162-262) */
   const long long *pre_ord; /* with pre: radial-cut survivors before each record */
