@@ -21,17 +21,18 @@
  * (-1)^(l+m) lambda_lm(theta) pairs each northern ring with its southern mirror.
  *
  * GPU layout:
- *   k_ring_phases  one block per (northern ring, 256 values of m).  Both hemispheres'
- *                  rings and both maps are staged through shared memory.  Each thread
- *                  sums one m, with twiddles stepped by complex multiplication and
- *                  re-seeded from an exact integer phase index every 1024 pixels.  It
- *                  writes S = F_north + F_south and D = F_north - F_south for each map,
- *                  laid out [m][ring] so that the next kernel reads one m's rings
- *                  contiguously.
- *   k_alm          one block per m; 8 rings per thread, recursion state in registers.
- *                  Per l the warp reduces its lanes' sums, and the block's warps are
- *                  summed in shared memory 64 values of l at a time.
- *   k_alm2cl       one thread per l.
+ *   rings     A ring's sums F_r(m) for all m are one FFT of its pixels.  Ring lengths are 4 n:
+ *             each ring pair (north and mirror) is split into its four interleaved quarters
+ *             of n pixels, for the sums S = north + south and the differences
+ *             D = north - south, with both maps in one complex sequence (a + i b).
+ *             k_quarter_fft transforms the quarters in shared memory: radix 2 when n is a
+ *             power of two (all belt rings), Bluestein's chirp convolution otherwise
+ *             (k_chirp prepares each cap ring's chirp transform), in two halves where its
+ *             length is over QF_MAX_CONV.  k_ring_combine joins the quarters for every m, separates the
+ *             maps and writes S and D of each map, laid out [m][ring] so that the next
+ *             kernel reads one m's rings contiguously.
+ *   k_alm     one block per m: rings over the threads, see there.
+ *   k_alm2cl  32 values of l by 32 slices of m per block.
  * All arithmetic is FP64: the estimator is a diagnostic, where exactness matters more
  * than speed.
  *
@@ -47,6 +48,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <vector>
@@ -58,12 +60,14 @@ namespace {
 
 #define FULL_MASK 0xffffffffu
 
-constexpr int RP_THREADS = 256; /* values of m per k_ring_phases block */
-constexpr int RP_CHUNK = 1024;  /* ring pixels staged per pass */
+constexpr int QF_THREADS = 256;
+constexpr int QF_MAX_CONV = 8192; /* longest transform in shared memory (128 KB) */
+constexpr int RC_THREADS = 256;
 constexpr int ALM_THREADS = 256;
 constexpr int ALM_RINGS = 8; /* rings per thread */
 constexpr int ALM_GROUP = ALM_THREADS * ALM_RINGS;
-constexpr int ALM_LC = 64; /* values of l per reduction chunk */
+constexpr int ALM_LC = 64; /* values of l between rescalings */
+constexpr int ALM_LB = 8;  /* values of l summed before a warp reduces them together */
 constexpr int ALM_WARPS = ALM_THREADS / 32;
 constexpr int FFT_THREADS = 512;
 constexpr int FFT_MAX_POW2 = 8192;
@@ -95,68 +99,225 @@ __device__ RingGeom ring_geom(int nside, int ith) {
   return g;
 }
 
+/* the same without z and sin(theta) */
+__device__ __forceinline__ RingGeom ring_geom_int(int nside, int ith) {
+  RingGeom g;
+  g.cth = g.sth = 0.0;
+  const bool cap = ith < nside;
+  g.nph = 4 * (cap ? ith : nside);
+  g.shift = cap ? 1 : (ith + 1 - nside) & 1;
+  g.start = cap ? 2LL * ith * (ith - 1)
+                : 2LL * nside * (nside - 1) + (long long)(ith - nside) * g.nph;
+  return g;
+}
+
 /* 2^(100 s) for |s| <= 10, zero below (the scales that underflow) */
 __device__ __forceinline__ double scale_factor(int s) {
   return (s < -10 || s > 10) ? 0.0 : ldexp(1.0, 100 * s);
 }
 
-/* F_r(m) of northern ring blockIdx.x + 1 and its mirror, for both maps */
-__global__ void __launch_bounds__(RP_THREADS)
-    k_ring_phases(const float *__restrict__ ma, const float *__restrict__ mb, int nside,
-                  int lmax, double *__restrict__ ph) {
-  __shared__ double sp[4][RP_CHUNK]; /* a north, a south, b north, b south */
-  const int ith = blockIdx.x + 1;
-  const int nrings = 2 * nside;
-  const RingGeom g = ring_geom(nside, ith);
-  const long long npix = 12LL * nside * nside;
-  const long long sn = g.start, ss = npix - g.start - g.nph;
-  const bool south = ith < nrings; /* the equator has no mirror */
-  const int m = blockIdx.y * RP_THREADS + threadIdx.x;
-  const bool act = m <= lmax;
-  const int nph = g.nph, period = 2 * nph;
-  /* exp(-i m phi_j) with phi_j = pi (2j + shift) / nph: phase index m (2j + shift)
-     mod 2 nph, and m enters only modulo 2 nph */
-  const long long mr = act ? (long long)(m % period) : 0;
-  double st_s, st_c;
-  sincospi((double)((2 * mr) % period) / (double)nph, &st_s, &st_c);
-  const double step_r = st_c, step_i = -st_s;
-  double ar[4] = {0.0, 0.0, 0.0, 0.0}, ai[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int j0 = 0; j0 < nph; j0 += RP_CHUNK) {
-    const int nj = min(RP_CHUNK, nph - j0);
-    __syncthreads();
-    for (int j = threadIdx.x; j < nj; j += RP_THREADS) {
-      sp[0][j] = (double)ma[sn + j0 + j];
-      sp[1][j] = south ? (double)ma[ss + j0 + j] : 0.0;
-      sp[2][j] = mb ? (double)mb[sn + j0 + j] : 0.0;
-      sp[3][j] = (mb && south) ? (double)mb[ss + j0 + j] : 0.0;
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+/* exp(-i pi a / n) for 0 <= a < 2 n */
+__device__ __forceinline__ double2 expi(long long a, int n) {
+  double s, c;
+  sincospi((double)a / (double)n, &s, &c);
+  return make_double2(c, -s);
+}
+
+/* length of the convolution that carries a DFT of length n (power of two >= 2 n - 1), or 0
+   when n is a power of two itself */
+__host__ __device__ __forceinline__ int conv_len(int n) {
+  if ((n & (n - 1)) == 0) return 0;
+  int l = 1;
+  while (l < 2 * n - 1) l <<= 1;
+  return l;
+}
+
+/* In-place radix-2 FFT of the len complex values in shared memory (len a power of two) by the
+   whole block, input in bit-reversed order.  tw[k] = exp(-2 pi i k / twlen), twlen >= len. */
+__device__ void block_fft(double2 *sz, int len, const double2 *__restrict__ tw, int twlen) {
+  for (int half = 1; half < len; half <<= 1) {
+    const int stride = twlen / (2 * half);
+    for (int b = threadIdx.x; b < len / 2; b += blockDim.x) {
+      const int pos = b & (half - 1);
+      const int i0 = ((b - pos) << 1) + pos, i1 = i0 + half;
+      const double2 u = sz[i0], t = cmul(sz[i1], tw[pos * stride]);
+      sz[i0] = make_double2(u.x + t.x, u.y + t.y);
+      sz[i1] = make_double2(u.x - t.x, u.y - t.y);
     }
     __syncthreads();
-    if (!act) continue;
-    const long long k0 = (mr * (2LL * j0 + g.shift)) % period;
-    double ws, wc;
-    sincospi((double)k0 / (double)nph, &ws, &wc);
-    double wr = wc, wi = -ws;
-    for (int j = 0; j < nj; j++) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        ar[q] = fma(sp[q][j], wr, ar[q]);
-        ai[q] = fma(sp[q][j], wi, ai[q]);
-      }
-      const double nr = wr * step_r - wi * step_i;
-      wi = fma(wr, step_i, wi * step_r);
-      wr = nr;
-    }
   }
-  if (!act) return;
-  double *o = ph + ((size_t)m * nrings + (ith - 1)) * 8;
-  o[0] = ar[0] + ar[1];
-  o[1] = ai[0] + ai[1];
-  o[2] = ar[0] - ar[1];
-  o[3] = ai[0] - ai[1];
-  o[4] = ar[2] + ar[3];
-  o[5] = ai[2] + ai[3];
-  o[6] = ar[2] - ar[3];
-  o[7] = ai[2] - ai[3];
+}
+__device__ __forceinline__ int bitrev(int j, int log2len) {
+  return log2len ? (int)(__brev((unsigned)j) >> (32 - log2len)) : 0;
+}
+
+/* A convolution longer than QF_MAX_CONV (16384, for n > 4096) goes as two transforms of half
+   its length: the even outputs of a transform of x are those of x_lo + x_hi, the odd ones
+   those of (x_lo - x_hi) w^j, w = exp(-2 pi i / conv); and of the inverse transform the first
+   half is the even inputs' plus w^-j times the odd inputs'. */
+__host__ __device__ __forceinline__ int conv_halves(int conv) { return conv > QF_MAX_CONV ? 2 : 1; }
+
+/* Bluestein's chirp of cap ring n = blockIdx.x + 1: the transform of the circular sequence
+   exp(+i pi j^2 / n), |j| < n, at chirp + off[n] (even outputs, then odd ones, where it is
+   made in halves); rings whose n is a power of two have none (off < 0) */
+__global__ void __launch_bounds__(QF_THREADS)
+    k_chirp(const long long *__restrict__ off, const double2 *__restrict__ tw, int twlen,
+            double2 *__restrict__ chirp) {
+  extern __shared__ double2 sz[];
+  const int n = blockIdx.x + 1;
+  if (off[n] < 0) return;
+  const int conv = conv_len(n), halves = conv_halves(conv), len = conv / halves;
+  const int lg = 31 - __clz(len);
+  auto value = [&](int j) {
+    const int a = j < n ? j : conv - j; /* circular distance from 0 */
+    double2 v = make_double2(0.0, 0.0);
+    if (a < n) {
+      v = expi(((long long)a * a) % (2 * n), n);
+      v.y = -v.y;
+    }
+    return v;
+  };
+  for (int h = 0; h < halves; h++) {
+    for (int j = threadIdx.x; j < len; j += blockDim.x) {
+      double2 v = value(j);
+      if (halves == 2) {
+        const double2 u = value(j + len);
+        v = h ? cmul(make_double2(v.x - u.x, v.y - u.y), tw[j * (twlen / conv)])
+              : make_double2(v.x + u.x, v.y + u.y);
+      }
+      sz[bitrev(j, lg)] = v;
+    }
+    __syncthreads();
+    block_fft(sz, len, tw, twlen);
+    for (int j = threadIdx.x; j < len; j += blockDim.x) chirp[off[n] + h * len + j] = sz[j];
+    __syncthreads();
+  }
+}
+
+/* Transform of one quarter: blockIdx.y = 2 q + type (type 0: S, 1: D), northern ring
+   blockIdx.x + 1 with its mirror, pixels 4 j + q, j < n:
+   G(k) = sum_j z_j exp(-2 pi i j k / n) at g + 8 start + (2 q + type) n, where start is the
+   first quarter-pixel of the ring (sum of the n of the rings before).  Latency of the
+   log2(n) passes and of the pixel loads bounds it: 8 blocks per ring keep every SM busy.  The
+   FP64 work is 5 n log2(n) against the 8 n (lmax + 1) of summing every m by itself.  Two maps
+   at Nside 512, lmax 1535: 0.84 ms, with k_chirp 0.08 and k_ring_combine 0.44, against 48.8 ms. */
+__global__ void __launch_bounds__(QF_THREADS)
+    k_quarter_fft(const float *__restrict__ ma, const float *__restrict__ mb, int nside,
+                  const long long *__restrict__ off, const double2 *__restrict__ chirp,
+                  const double2 *__restrict__ tw, int twlen, double2 *__restrict__ g) {
+  extern __shared__ double2 sz[];
+  const int ith = blockIdx.x + 1, q = blockIdx.y >> 1;
+  const double sgn = (blockIdx.y & 1) ? -1.0 : 1.0;
+  const RingGeom rg = ring_geom_int(nside, ith);
+  const int n = rg.nph >> 2;
+  const long long npix = 12LL * nside * nside;
+  const long long sn = rg.start + q, ss = npix - rg.start - rg.nph + q;
+  const bool south = ith < 2 * nside; /* the equator has no mirror */
+  double2 *out = g + (rg.start >> 2) * 8 + (long long)blockIdx.y * n;
+  auto pixel = [&](int j) {
+    double2 z = make_double2((double)ma[sn + 4 * j], mb ? (double)mb[sn + 4 * j] : 0.0);
+    if (south) {
+      z.x = fma(sgn, (double)ma[ss + 4 * j], z.x);
+      if (mb) z.y = fma(sgn, (double)mb[ss + 4 * j], z.y);
+    }
+    return z;
+  };
+  const int conv = conv_len(n);
+  if (conv == 0) {
+    const int lg = 31 - __clz(n);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) sz[bitrev(j, lg)] = pixel(j);
+    __syncthreads();
+    block_fft(sz, n, tw, twlen);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) out[j] = sz[j];
+    return;
+  }
+  /* DFT(k) = c_k sum_j (z_j c_j) conj(c_{k-j}), c_j = exp(-i pi j^2 / n): a circular
+     convolution; its inverse transform as the conjugate of a forward one */
+  const int halves = conv_halves(conv), len = conv / halves, lg = 31 - __clz(len);
+  const double inv = 1.0 / (double)conv;
+  for (int h = 0; h < halves; h++) {
+    for (int j = threadIdx.x; j < len; j += blockDim.x) {
+      double2 v = make_double2(0.0, 0.0);
+      if (j < n) v = cmul(pixel(j), expi(((long long)j * j) % (2 * n), n));
+      if (h) v = cmul(v, tw[j * (twlen / conv)]);
+      sz[bitrev(j, lg)] = v;
+    }
+    __syncthreads();
+    block_fft(sz, len, tw, twlen);
+    const double2 *ch = chirp + off[n] + h * len;
+    /* product, conjugated, into bit-reversed order (pairs swapped in place) */
+    for (int j = threadIdx.x; j < len; j += blockDim.x) {
+      const int r = bitrev(j, lg);
+      if (r < j) continue;
+      double2 a = cmul(sz[j], ch[j]);
+      a.y = -a.y;
+      if (r != j) {
+        double2 b = cmul(sz[r], ch[r]);
+        b.y = -b.y;
+        sz[j] = b;
+      }
+      sz[r] = a;
+    }
+    __syncthreads();
+    block_fft(sz, len, tw, twlen);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      double2 v = make_double2(sz[j].x * inv, -sz[j].y * inv);
+      if (h) {
+        const double2 w = tw[j * (twlen / conv)];
+        v = cmul(v, make_double2(w.x, -w.y));
+      }
+      v = cmul(v, expi(((long long)j * j) % (2 * n), n));
+      out[j] = h ? make_double2(out[j].x + v.x, out[j].y + v.y) : v;
+    }
+    __syncthreads();
+  }
+}
+
+/* F_r(m), m = blockIdx.y * RC_THREADS + thread, of northern ring blockIdx.x + 1 with its mirror:
+   Z(k) = sum_q w^(k q) G_q(k mod n) with w = exp(-2 pi i / 4n), k = m mod 4n, times the ring's
+   half-pixel phase; the maps a and b of z = a + i b come apart as (Z(k) +- conj Z(-k)) / 2.
+   ph[m][ring] = S and D of map a, then of map b. */
+__global__ void __launch_bounds__(RC_THREADS)
+    k_ring_combine(const double2 *__restrict__ g, int nside, int lmax, double *__restrict__ ph) {
+  const int ith = blockIdx.x + 1, m = blockIdx.y * RC_THREADS + threadIdx.x;
+  if (m > lmax) return;
+  const RingGeom rg = ring_geom_int(nside, ith);
+  const int nph = rg.nph, n = nph >> 2;
+  const double2 half = expi(m % (2 * nph), nph); /* exp(-i pi m / nph) */
+  const double2 w1 = cmul(half, half), w2 = cmul(w1, w1), w3 = cmul(w2, w1);
+  const int kp = m % n, km = kp ? n - kp : 0;
+  const double2 *src = g + (rg.start >> 2) * 8;
+  double o[8];
+#pragma unroll
+  for (int type = 0; type < 2; type++) {
+    double2 zp = src[type * n + kp], zm = src[type * n + km];
+#pragma unroll
+    for (int q = 1; q < 4; q++) {
+      const double2 w = q == 1 ? w1 : q == 2 ? w2 : w3;
+      const double2 a = cmul(src[(2 * q + type) * n + kp], w);
+      const double2 b = cmul(src[(2 * q + type) * n + km], make_double2(w.x, -w.y));
+      zp.x += a.x;
+      zp.y += a.y;
+      zm.x += b.x;
+      zm.y += b.y;
+    }
+    double2 fa = make_double2(0.5 * (zp.x + zm.x), 0.5 * (zp.y - zm.y));
+    double2 fb = make_double2(0.5 * (zp.y + zm.y), 0.5 * (zm.x - zp.x));
+    if (rg.shift) {
+      fa = cmul(fa, half);
+      fb = cmul(fb, half);
+    }
+    o[2 * type] = fa.x;
+    o[2 * type + 1] = fa.y;
+    o[4 + 2 * type] = fb.x;
+    o[4 + 2 * type + 1] = fb.y;
+  }
+  double2 *dst = (double2 *)(ph + ((size_t)m * (2 * nside) + (ith - 1)) * 8);
+#pragma unroll
+  for (int c = 0; c < 4; c++) dst[c] = make_double2(o[2 * c], o[2 * c + 1]);
 }
 
 /* row offset of m in the packed a_lm array (l = m .. lmax) */
@@ -164,38 +325,62 @@ __host__ __device__ __forceinline__ size_t alm_row(int m, int lmax) {
   return (size_t)m * (size_t)(lmax + 1) - (size_t)m * (size_t)(m - 1) / 2;
 }
 
-/* a_lm / omega_pix of both maps for m = blockIdx.x, added into alm[(row + l - m) * 4 + c],
-   c = (Re a, Im a, Re b, Im b) */
+/* sums of v[32] over the warp's lanes: lane i returns the sum of the lanes' v[i].  Each step
+   halves the values a lane holds, so 32 values take 31 additions, not 160. */
+__device__ __forceinline__ double warp_sum32(double (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; i++) {
+      const double mine = up ? v[i + o] : v[i], other = up ? v[i] : v[i + o];
+      v[i] = mine + __shfl_xor_sync(FULL_MASK, other, o);
+    }
+  }
+  return v[0];
+}
+
+/* a_lm / omega_pix of both maps for m = blockIdx.x, in alm[(row + l - m) * 4 + c],
+   c = (Re a, Im a, Re b, Im b), which starts at zero.
+   TWO: there is a map b (its c stay zero otherwise).
+
+   FP64 issue bounds it (2 operations per clock and SM).  The recursion is carried without the
+   normalising factors: lambda_l = C_l q_l with q_{l+1} = cos(theta) q_l - beta_l q_{l-1},
+   beta_l = (l^2 - m^2) / (4 l^2 - 1) and C_l the product of rf(j) = 1 / sqrt(beta_{j+1}),
+   j < l, which is applied once per l to the sum over the rings.  A ring's scale (the powers of
+   2^100 and lambda_mm) is applied to its phases, and q is looked over for rescaling, every 64
+   values of l, over which it changes by less than 2^310.  So a ring and l cost 2 operations of
+   recursion and 2 per map for the sums.  Rings that l_min_ylm leaves out for every l are
+   skipped a warp at a time, and the sums of 64 values of l below it too.  Nside 512, lmax
+   1535, two maps: 14.3 ms (6 operations for each of 1.2e9 rings and l are 11.9 ms), against
+   48.8 ms with every factor and test at every l. */
+template <bool TWO>
 __global__ void __launch_bounds__(ALM_THREADS)
     k_alm(const double *__restrict__ ph, const double *__restrict__ mfac, int nside, int lmax,
-          double *__restrict__ alm) {
+          int group, double *__restrict__ alm) {
   extern __shared__ double smem[];
-  double *sph = smem;                 /* [ALM_GROUP][8] phases of this m */
-  double *rfa = sph + ALM_GROUP * 8;  /* rf(l), l = l0 .. l0 + LC - 1 */
-  double *rfb = rfa + ALM_LC;         /* 1 / rf(l - 1) */
-  double *red = rfb + ALM_LC;         /* [warp][LC][4] */
+  constexpr int NC = TWO ? 4 : 2;     /* sums per l */
+  double *sph = smem;                 /* [component 8][group] phases, times the ring's scale */
+  double *beta = sph + group * 8;     /* beta_l, l = l0 .. l0 + LC - 1 */
+  double *cl = beta + ALM_LC;         /* C_l / C_l0 */
+  double *red = cl + ALM_LC;          /* [warp][LC][4] */
   const int m = blockIdx.x;
   const int nrings = 2 * nside;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const double dm2 = (double)m * (double)m;
   const size_t row = alm_row(m, lmax);
   const double mf = mfac[m];
-  for (int g0 = 0; g0 < nrings; g0 += ALM_GROUP) {
-    const int ng = min(ALM_GROUP, nrings - g0);
-    __syncthreads();
-    const double *src = ph + ((size_t)m * nrings + g0) * 8;
-    for (int i = t; i < ng * 8; i += ALM_THREADS) sph[i] = src[i];
-    double cth[ALM_RINGS], lprev[ALM_RINGS], lcur[ALM_RINGS], cm[ALM_RINGS], lmm[ALM_RINGS];
+  for (int g0 = 0; g0 < nrings; g0 += group) {
+    const int ng = min(group, nrings - g0);
+    const int nk = (ng + ALM_THREADS - 1) / ALM_THREADS;
+    double cth[ALM_RINGS], qp[ALM_RINGS], qc[ALM_RINGS], lmm[ALM_RINGS];
     int sc[ALM_RINGS], lmin[ALM_RINGS];
-    int any = 0;
+    unsigned alive = 0; /* bit k: some ring of this warp's k-th 32 is used */
 #pragma unroll
     for (int k = 0; k < ALM_RINGS; k++) {
       const int r = k * ALM_THREADS + t;
-      cth[k] = 0.0;
-      lprev[k] = 0.0;
-      lcur[k] = 0.0;
-      cm[k] = 0.0;
-      lmm[k] = 0.0;
+      cth[k] = qp[k] = qc[k] = lmm[k] = 0.0;
       sc[k] = 0;
       lmin[k] = INT_MAX;
       if (r < ng) {
@@ -209,107 +394,160 @@ __global__ void __launch_bounds__(ALM_THREADS)
           double lam_mm = exp2(log2val - 100.0 * (double)s);
           if (m & 1) lam_mm = -lam_mm;
           cth[k] = gg.cth;
-          lcur[k] = 1.0; /* lambda_m / (lambda_mm scale) */
+          qc[k] = 1.0; /* lambda_m / (lambda_mm scale) */
           lmm[k] = lam_mm;
           sc[k] = s;
-          cm[k] = scale_factor(s) * lam_mm;
           lmin[k] = lm;
-          any = 1;
         }
       }
+      if (__any_sync(FULL_MASK, lmin[k] <= lmax)) alive |= 1u << k;
     }
-    if (!__syncthreads_or(any)) continue;
+    if (!__syncthreads_or(alive != 0)) continue;
+    double c_run = 1.0; /* C_l0, its power of two moved into q */
+    bool first = true;
     for (int l0 = m; l0 <= lmax; l0 += ALM_LC) {
-      __syncthreads();
+      const int nl = min(ALM_LC, lmax - l0 + 1);
+      /* beta_l, and the factors 1 / sqrt(beta_{l+1}) of C */
       if (t < ALM_LC) {
-        /* gen_recfac: rf(l) = sqrt((4 (l+1)^2 - 1) / ((l+1)^2 - m^2)) */
         const int l = l0 + t;
-        const double f1 = (double)(l + 1) * (double)(l + 1);
-        rfa[t] = sqrt((4.0 * f1 - 1.0) / (f1 - dm2));
-        if (l - 1 >= m) {
-          const double f0 = (double)l * (double)l;
-          rfb[t] = 1.0 / sqrt((4.0 * f0 - 1.0) / (f0 - dm2));
-        } else {
-          rfb[t] = 0.0;
+        const double f0 = (double)l * (double)l, f1 = (double)(l + 1) * (double)(l + 1);
+        beta[t] = l > m ? (f0 - dm2) / (4.0 * f0 - 1.0) : 0.0;
+        double p = sqrt((4.0 * f1 - 1.0) / (f1 - dm2)); /* rf(l): C_{l+1} / C_l */
+        /* inclusive product over the 32 lanes, then the second warp takes the first's */
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(FULL_MASK, p, o);
+          if (lane >= o) p *= y;
+        }
+        cl[t] = p;
+      }
+      /* the rings' scales and rescaling */
+      int lcut = INT_MAX; /* smallest l_min of this lane's rings */
+#pragma unroll
+      for (int k = 0; k < ALM_RINGS; k++) {
+        if (k >= nk || !((alive >> k) & 1u)) continue;
+        double a = fmax(fabs(qc[k]), fabs(qp[k]));
+        bool moved = first;
+        while (a > 0x1p100) {
+          qp[k] *= 0x1p-100;
+          qc[k] *= 0x1p-100;
+          a *= 0x1p-100;
+          sc[k] += 1;
+          moved = true;
+        }
+        while (a < 0x1p-100 && a != 0.0) {
+          qp[k] *= 0x1p100;
+          qc[k] *= 0x1p100;
+          a *= 0x1p100;
+          sc[k] -= 1;
+          moved = true;
+        }
+        lcut = min(lcut, lmin[k]);
+        const int r = k * ALM_THREADS + t;
+        if (r < ng && moved) {
+          const double cm = scale_factor(sc[k]) * lmm[k];
+          const double2 *src = (const double2 *)(ph + ((size_t)m * nrings + g0 + r) * 8);
+#pragma unroll
+          for (int c = 0; c < (TWO ? 4 : 2); c++) {
+            const double2 f = cm != 0.0 ? src[c] : make_double2(0.0, 0.0);
+            sph[(2 * c) * group + r] = f.x * cm;
+            sph[(2 * c + 1) * group + r] = f.y * cm;
+          }
         }
       }
+      first = false;
+      const bool sums = __any_sync(FULL_MASK, lcut < l0 + nl);
       __syncthreads();
-      const int nl = min(ALM_LC, lmax - l0 + 1);
-      for (int i = 0; i < nl; i++) {
-        const int l = l0 + i;
-        const int par = ((l + m) & 1) ? 2 : 0; /* S for even l + m, D for odd */
-        const double ra = rfa[i], rb = rfb[i];
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      if (t >= 32 && t < ALM_LC) cl[t] *= cl[31];
+      __syncthreads();
+      for (int i0 = 0; i0 < nl; i0 += ALM_LB) {
+        double acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; i++) acc[i] = 0.0;
+        const int par = (l0 + i0 + m) & 1; /* S for even l + m, D for odd */
+        double b[ALM_LB];
+#pragma unroll
+        for (int i = 0; i < ALM_LB; i++) b[i] = beta[i0 + i];
 #pragma unroll
         for (int k = 0; k < ALM_RINGS; k++) {
-          if (l >= lmin[k]) {
-            const double lam = lcur[k] * cm[k];
-            const double *p = sph + (size_t)(k * ALM_THREADS + t) * 8;
-            s0 = fma(lam, p[par], s0);
-            s1 = fma(lam, p[par + 1], s1);
-            s2 = fma(lam, p[4 + par], s2);
-            s3 = fma(lam, p[5 + par], s3);
-          }
-          /* lambda_{l+1} = rf(l) (cos theta lambda_l - lambda_{l-1} / rf(l-1)) */
-          const double back = lprev[k] * rb;
-          lprev[k] = lcur[k];
-          const double nx = (cth[k] * lcur[k] - back) * ra;
-          lcur[k] = nx;
-          if (fabs(nx) > 0x1p100) {
-            lprev[k] *= 0x1p-100;
-            lcur[k] *= 0x1p-100;
-            sc[k] += 1;
-            cm[k] = scale_factor(sc[k]) * lmm[k];
-          } else if (fabs(nx) < 0x1p-100 && nx != 0.0) {
-            lprev[k] *= 0x1p100;
-            lcur[k] *= 0x1p100;
-            sc[k] -= 1;
-            cm[k] = scale_factor(sc[k]) * lmm[k];
-          }
-        }
+          if (k >= nk || !((alive >> k) & 1u)) continue;
+          const int r = k * ALM_THREADS + t;
+          double f[2][NC];
+          if (sums) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          s0 += __shfl_xor_sync(FULL_MASK, s0, o);
-          s1 += __shfl_xor_sync(FULL_MASK, s1, o);
-          s2 += __shfl_xor_sync(FULL_MASK, s2, o);
-          s3 += __shfl_xor_sync(FULL_MASK, s3, o);
+            for (int c = 0; c < NC; c++) {
+              const int comp = (c >> 1) * 4 + (c & 1);
+              f[0][c] = r < ng ? sph[(comp + 2 * par) * group + r] : 0.0;
+              f[1][c] = r < ng ? sph[(comp + 2 - 2 * par) * group + r] : 0.0;
+            }
+          }
+          double x0 = qp[k], x1 = qc[k];
+#pragma unroll
+          for (int i = 0; i < ALM_LB; i++) {
+            if (sums) {
+#pragma unroll
+              for (int c = 0; c < NC; c++) acc[i * 4 + c] = fma(x1, f[i & 1][c], acc[i * 4 + c]);
+            }
+            /* q_{l+1}; past the last l of the chunk its values are not used */
+            const double nx = fma(cth[k], x1, -b[i] * x0);
+            x0 = x1;
+            x1 = nx;
+          }
+          qp[k] = x0;
+          qc[k] = x1;
         }
-        if (lane == 0) {
-          double *q = red + ((size_t)w * ALM_LC + i) * 4;
-          q[0] = s0;
-          q[1] = s1;
-          q[2] = s2;
-          q[3] = s3;
-        }
+        const double s = sums ? warp_sum32(acc) : 0.0;
+        red[(w * ALM_LC + i0) * 4 + lane] = s;
       }
       __syncthreads();
       if (t < nl * 4) {
         const int i = t >> 2, c = t & 3;
         double s = 0.0;
         for (int ww = 0; ww < ALM_WARPS; ww++) s += red[((size_t)ww * ALM_LC + i) * 4 + c];
+        s *= i ? c_run * cl[i - 1] : c_run;
         alm[(row + (size_t)(l0 + i - m)) * 4 + c] += s;
       }
+      /* C of the next chunk, its power of two moved into q */
+      int e = 0;
+      c_run = frexp(c_run * cl[ALM_LC - 1], &e);
+      const double up = ldexp(1.0, e);
+#pragma unroll
+      for (int k = 0; k < ALM_RINGS; k++) {
+        qp[k] *= up;
+        qc[k] *= up;
+      }
+      __syncthreads();
     }
   }
 }
 
-/* alm2cl: cl[0] a x a, cl[1] a x b, cl[2] b x b, each [lmax + 1] */
-__global__ void k_alm2cl(const double *__restrict__ alm, int lmax, double omega2,
-                         double *__restrict__ cl) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l > lmax) return;
+/* alm2cl: cl[0] a x a, cl[1] a x b, cl[2] b x b, each [lmax + 1].  32 values of l (one per
+   lane: their a_lm are contiguous) by 32 slices of m, summed in a fixed order */
+__global__ void __launch_bounds__(1024)
+    k_alm2cl(const double *__restrict__ alm, int lmax, double omega2, double *__restrict__ cl) {
+  __shared__ double part[3][32][33];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int l = blockIdx.x * 32 + lane;
   double aa = 0.0, ab = 0.0, bb = 0.0;
-  for (int m = 1; m <= l; m++) {
-    const double *a = alm + (alm_row(m, lmax) + (size_t)(l - m)) * 4;
-    aa += a[0] * a[0] + a[1] * a[1];
-    ab += a[0] * a[2] + a[1] * a[3];
-    bb += a[2] * a[2] + a[3] * a[3];
-  }
+  if (l <= lmax)
+    for (int m = 1 + slice; m <= l; m += 32) {
+      const double2 *a = (const double2 *)(alm + (alm_row(m, lmax) + (size_t)(l - m)) * 4);
+      const double2 x = a[0], y = a[1];
+      aa += x.x * x.x + x.y * x.y;
+      ab += x.x * y.x + x.y * y.y;
+      bb += y.x * y.x + y.y * y.y;
+    }
+  part[0][slice][lane] = aa;
+  part[1][slice][lane] = ab;
+  part[2][slice][lane] = bb;
+  __syncthreads();
+  if (slice >= 3 || l > lmax) return;
+  double s = 0.0;
+  for (int i = 0; i < 32; i++) s += part[slice][i][lane];
   const double *a0 = alm + (size_t)l * 4; /* m = 0 */
-  const double inv = omega2 / (2.0 * (double)l + 1.0);
-  cl[l] = (2.0 * aa + (a0[0] * a0[0] - a0[1] * a0[1])) * inv;
-  cl[lmax + 1 + l] = (2.0 * ab + (a0[0] * a0[2] - a0[1] * a0[3])) * inv;
-  cl[2 * (lmax + 1) + l] = (2.0 * bb + (a0[2] * a0[2] - a0[3] * a0[3])) * inv;
+  const double z = slice == 0   ? a0[0] * a0[0] - a0[1] * a0[1]
+                   : slice == 1 ? a0[0] * a0[2] - a0[1] * a0[3]
+                                : a0[2] * a0[2] - a0[3] * a0[3];
+  cl[(size_t)slice * (lmax + 1) + l] = (2.0 * s + z) * (omega2 / (2.0 * (double)l + 1.0));
 }
 
 /* ------------------------------------------------------------------ flat sky ---- */
@@ -517,17 +755,57 @@ int32_t p2m_cl_healpix(int32_t device, const float *map_a, const float *map_b, i
     SP_CK(cudaMemcpyAsync(d_b, map_b, sizeof(float) * (size_t)npix, cudaMemcpyHostToDevice, st.s));
   SP_CK(cudaMemcpyAsync(d_mfac, mfac.data(), sizeof(double) * mfac.size(), cudaMemcpyHostToDevice,
                         st.s));
-  SP_CK(cudaMemsetAsync(d_alm, 0, sizeof(double) * 4 * nalm, st.s));
-  k_ring_phases<<<dim3(nrings, (lmax + RP_THREADS) / RP_THREADS), RP_THREADS, 0, st.s>>>(
-      d_a, d_b, nside, lmax, d_ph);
+  /* the cap rings' chirps: offsets by n = 1 .. nside - 1, -1 where none is used */
+  std::vector<long long> off((size_t)nside + 1, -1);
+  long long nchirp = 0;
+  int twlen = nside, longest = nside; /* longest transform; longest piece in shared memory */
+  for (int n = 1; n < nside; n++) {
+    const int len = conv_len(n);
+    if (len == 0) continue;
+    off[(size_t)n] = nchirp;
+    nchirp += len;
+    twlen = std::max(twlen, len);
+    longest = std::max(longest, len / conv_halves(len));
+  }
+  double2 *d_tw = nullptr, *d_chirp = nullptr, *d_g = nullptr;
+  long long *d_off = nullptr;
+  SP_CK(B.get(&d_tw, sizeof(double2) * (size_t)(twlen / 2 + 1)));
+  SP_CK(B.get(&d_chirp, sizeof(double2) * (size_t)nchirp));
+  SP_CK(B.get(&d_off, sizeof(long long) * off.size()));
+  /* quarters of all northern rings (2 nside (nside - 1) + 4 nside (nside + 1) pixels), S and D */
+  const long long north = 2LL * nside * (nside - 1) + 4LL * nside * (nside + 1);
+  SP_CK(B.get(&d_g, sizeof(double2) * 2 * (size_t)north));
+  SP_CK(cudaMemcpyAsync(d_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice,
+                        st.s));
+  k_twiddles<<<(twlen / 2 + 256) / 256, 256, 0, st.s>>>(d_tw, twlen);
   SP_CK(cudaGetLastError());
-  const size_t smem = sizeof(double) * ((size_t)ALM_GROUP * 8 + 2 * ALM_LC +
+  const size_t fsmem = sizeof(double2) * (size_t)longest;
+  SP_CK(cudaFuncSetAttribute(k_chirp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+  SP_CK(cudaFuncSetAttribute(k_quarter_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+  if (nside > 1) {
+    k_chirp<<<nside - 1, QF_THREADS, fsmem, st.s>>>(d_off, d_tw, twlen, d_chirp);
+    SP_CK(cudaGetLastError());
+  }
+  k_quarter_fft<<<dim3(nrings, 8), QF_THREADS, fsmem, st.s>>>(d_a, d_b, nside, d_off, d_chirp, d_tw,
+                                                              twlen, d_g);
+  SP_CK(cudaGetLastError());
+  k_ring_combine<<<dim3(nrings, (lmax + RC_THREADS) / RC_THREADS), RC_THREADS, 0, st.s>>>(
+      d_g, nside, lmax, d_ph);
+  SP_CK(cudaGetLastError());
+  SP_CK(cudaMemsetAsync(d_alm, 0, sizeof(double) * 4 * nalm, st.s));
+  const int group = std::min(ALM_GROUP, (nrings + ALM_THREADS - 1) / ALM_THREADS * ALM_THREADS);
+  const size_t smem = sizeof(double) * ((size_t)group * 8 + 2 * ALM_LC +
                                         (size_t)ALM_WARPS * ALM_LC * 4);
-  SP_CK(cudaFuncSetAttribute(k_alm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_alm<<<lmax + 1, ALM_THREADS, smem, st.s>>>(d_ph, d_mfac, nside, lmax, d_alm);
+  if (map_b) {
+    SP_CK(cudaFuncSetAttribute(k_alm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_alm<true><<<lmax + 1, ALM_THREADS, smem, st.s>>>(d_ph, d_mfac, nside, lmax, group, d_alm);
+  } else {
+    SP_CK(cudaFuncSetAttribute(k_alm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_alm<false><<<lmax + 1, ALM_THREADS, smem, st.s>>>(d_ph, d_mfac, nside, lmax, group, d_alm);
+  }
   SP_CK(cudaGetLastError());
   const double omega = 4.0 * M_PI / (double)npix;
-  k_alm2cl<<<(lmax + 128) / 128, 128, 0, st.s>>>(d_alm, lmax, omega * omega, d_cl);
+  k_alm2cl<<<(lmax + 32) / 32, 1024, 0, st.s>>>(d_alm, lmax, omega * omega, d_cl);
   SP_CK(cudaGetLastError());
   std::vector<double> cl(3 * (size_t)(lmax + 1));
   SP_CK(cudaMemcpyAsync(cl.data(), d_cl, sizeof(double) * cl.size(), cudaMemcpyDeviceToHost, st.s));

@@ -54,3 +54,59 @@ def test_fp64_fast_path_equals_exact_path(nside, which, big_rings, monkeypatch):
         ulp = np.spacing(np.maximum(np.abs(a), np.abs(b)))
         assert np.all(np.abs(a.astype(np.float64) - b) <= ulp)
         assert np.mean(a != b) < 1e-4
+
+
+def first_pixel(nside, ring):
+    """(first pixel, pixels, longitude of the first) of a ring, from the RING layout."""
+    n, i = nside, min(ring, 4 * nside - ring)
+    npr = 4 * min(i, n)
+    if ring < n:
+        first, shift = 2 * ring * (ring - 1), 0.5
+    elif ring <= 3 * n:
+        first, shift = 2 * n * (n - 1) + (ring - n) * 4 * n, 0.5 * ((ring - n + 1) % 2)
+    else:
+        first, shift = 12 * n * n - 2 * i * (i + 1), 0.5
+    return first, npr, 2 * np.pi * shift / npr
+
+
+@pytest.mark.parametrize("two", [True, False])
+@pytest.mark.parametrize("nside,lmax", [(1, 4), (2, 7), (8, 20), (128, 131), (512, 64),
+                                        (2048, 66), (4096, 40), (8192, 17)])
+def test_sphere_spectra_of_sparse_maps(nside, lmax, two):
+    """Ring transforms of every kind (power-of-two rings, chirp convolutions in one piece and
+    in halves, rings of one quarter-pixel) and several groups of rings: maps that are zero but for
+    some pixels of a few rings, whose a_lm are short direct sums.  The direct sum and the
+    library round differently in each of ~l steps: 1e-10 of the largest C_l."""
+    import spectra
+    rng = np.random.default_rng(nside + lmax)
+    rings = sorted({1, 2, 3, nside - 1, nside, nside + 1, 2 * nside, 2 * nside + 1, 3 * nside + 1,
+                    4 * nside - 1, 4 * nside - 3, *rng.integers(1, 4 * nside, 12).tolist()}
+                   & set(range(1, 4 * nside)))
+    maps = np.zeros((2, 12 * nside * nside), dtype=np.float32)
+    alm = np.zeros((2, lmax + 1, lmax + 1), dtype=np.complex128)
+    thetas = np.array([spectra.healpix_rings(nside)[r - 1][0] for r in rings]) if nside <= 128 \
+        else np.array([np.arccos(ring_z(nside, r)) for r in rings])
+    lam = spectra._ylm_theta(lmax, thetas)
+    for k, ring in enumerate(rings):
+        first, npr, phi0 = first_pixel(nside, ring)
+        js = np.unique(rng.integers(0, npr, 5))
+        for q in range(2):
+            v = rng.standard_normal(js.size).astype(np.float32)
+            maps[q, first + js] = v
+            phase = np.exp(-1j * np.outer(np.arange(lmax + 1), phi0 + 2 * np.pi * js / npr)) @ v
+            alm[q] += lam[:, :, k] * phase
+    alm *= 4 * np.pi / maps.shape[1]
+    want = {"aa": spectra.cl_from_alm(alm[0], alm[0])}
+    if two:
+        want["ab"] = spectra.cl_from_alm(alm[0], alm[1])
+        want["bb"] = spectra.cl_from_alm(alm[1], alm[1])
+    got = p2m.cl_healpix(maps[0], maps[1] if two else None, lmax=lmax)
+    assert set(got) == set(want)
+    for key in want:
+        assert np.abs(got[key] - want[key]).max() <= 1e-10 * np.abs(want[key]).max()
+
+
+def ring_z(nside, ring):
+    i = min(ring, 4 * nside - ring)
+    z = 1 - i * i / (3.0 * nside * nside) if i < nside else (2 * nside - i) / (1.5 * nside)
+    return z if ring <= 2 * nside else -z
