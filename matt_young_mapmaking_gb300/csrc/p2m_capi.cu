@@ -74,8 +74,9 @@ struct p2m_ctx {
   float *d_out_own[P2M_MAXMAPS] = {};
   float *d_out[P2M_MAXMAPS] = {};
   double *d_acc64 = nullptr; /* full-sky FP64 accumulator (plain and FP64-accumulating paths) */
-  /* compensated path: the output maps accumulate the high words; low words and their
-     dirty-tile flags stay zero between sweeps */
+  /* compensated path: the output maps accumulate the high words; low words stay zero between
+     sweeps.  The flags of the tiles with a nonzero low word (compensated), or that may hold
+     sums (the others), do too */
   float *d_lo = nullptr;
   unsigned char *d_tiles = nullptr;
   bool outs_zeroed = false;
@@ -405,14 +406,15 @@ p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, long long n_max, cuda
 
 bool compensated(const p2m_ctx *ctx) { return ctx->d_lo != nullptr; }
 
-/* the compensated path accumulates into the output maps: clear them before the first
-   paint after a reset (the buffers bound at that time).  The clear is bandwidth-bound
-   and independent of the ingest, so it runs on a side stream after the work already on
-   s; the sweep waits for it before painting. */
+/* the output maps are cleared before the first paint after a reset (the buffers bound at that
+   time): the compensated path accumulates into them, the others' read-out adds the painted
+   tiles to them.  The clear is bandwidth-bound and independent of the ingest, so it runs on a
+   side stream after the work already on s; the compensated painting, or the others' read-out,
+   waits for it. */
 p2m_status wait_reads(p2m_ctx *ctx, cudaStream_t s);
 
 p2m_status zero_outputs(p2m_ctx *ctx, cudaStream_t s) {
-  if (!compensated(ctx) || ctx->outs_zeroed) return P2M_OK;
+  if (ctx->cfg.nside <= 0 || ctx->outs_zeroed) return P2M_OK;
   CK(cudaEventRecord(ctx->ev_zero_start, s));
   CK(cudaStreamWaitEvent(ctx->zstream, ctx->ev_zero_start, 0));
   ST(wait_reads(ctx, ctx->zstream));
@@ -639,7 +641,7 @@ SweepBuffers sweep_buffers(const p2m_ctx *ctx) {
    that turns them into maps is left to the next sweep */
 p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   ST(flush_prepared(ctx));
-  ST(wait_zero(ctx, s));
+  if (compensated(ctx)) ST(wait_zero(ctx, s));
   if (ctx->cfg.nside <= 0) {
     ctx->dirty = false;
     return P2M_OK;
@@ -657,7 +659,7 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
     CK(grow(&ctx->d_pix_off, &ctx->cap_pix_off, n));
     unsigned long long nn = (unsigned long long)n;
     CK(cudaMemcpyAsync(ctx->d_nitems, &nn, sizeof(nn), cudaMemcpyHostToDevice, s));
-    p2m_launch_item_counts(ctx->d_items_raw, n, ctx->d_counts, s, ctx->nsm);
+    p2m_launch_item_counts(P, sweep_buffers(ctx), ctx->d_counts, s, ctx->nsm);
     p2m_launch_scan_u32(ctx->d_counts, ctx->d_nitems, ctx->d_pix_off, &ctx->d_ctr->n_pix,
                         ctx->d_scan_tmp, s);
   }
@@ -702,6 +704,7 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
 p2m_status sweep(p2m_ctx *ctx, cudaStream_t s) {
   ST(paint_pending(ctx, s));
   if (ctx->cfg.nside <= 0) return P2M_OK;
+  ST(wait_zero(ctx, s));
   if (!ctx->unfolded) {
     if (!ctx->swept) {
       ST(wait_reads(ctx, s));
@@ -721,11 +724,9 @@ p2m_status sweep(p2m_ctx *ctx, cudaStream_t s) {
     /* fold the sparse low words into the maps and clear them */
     p2m_launch_fold_lo(P, W, s, ctx->nsm);
   } else {
-    /* the read-out reads the accumulator; a memset then clears it for the next paint */
-    p2m_launch_finalize_full(P, ctx->d_acc64, ctx->hp_npix, ctx->d_out, ctx->swept ? 1 : 0, s,
-                             ctx->nsm);
-    CK(cudaMemsetAsync(ctx->d_acc64, 0,
-                       sizeof(double) * (size_t)ctx->cfg.nmaps * (size_t)ctx->hp_npix, s));
+    /* the read-out reads the painted tiles; they are cleared after it for the next paint */
+    p2m_launch_read_tiles(P, W, ctx->swept ? 1 : 0, s, ctx->nsm);
+    p2m_launch_clear_tiles(P, W, s, ctx->nsm);
   }
   TE(PH_READOUT);
   CK(cudaGetLastError());
@@ -835,16 +836,16 @@ p2m_status p2m_create(const p2m_config *cfg, p2m_ctx **out) {
     }
     if (cfg->precision == P2M_PREC_MIXED) {
       size_t lb = sizeof(float) * (size_t)cfg->nmaps * (size_t)ctx->hp_npix;
-      size_t tb = (size_t)((ctx->hp_npix + P2M_TILE_PIX - 1) >> P2M_TILE_SHIFT);
       CK(cudaMalloc((void **)&ctx->d_lo, lb));
       CK(cudaMemset(ctx->d_lo, 0, lb));
-      CK(cudaMalloc((void **)&ctx->d_tiles, tb));
-      CK(cudaMemset(ctx->d_tiles, 0, tb));
     } else {
       size_t ab = sizeof(double) * (size_t)cfg->nmaps * (size_t)ctx->hp_npix;
       CK(cudaMalloc((void **)&ctx->d_acc64, ab));
       CK(cudaMemset(ctx->d_acc64, 0, ab));
     }
+    size_t tb = (size_t)((ctx->hp_npix + P2M_TILE_PIX - 1) >> P2M_TILE_SHIFT);
+    CK(cudaMalloc((void **)&ctx->d_tiles, tb));
+    CK(cudaMemset(ctx->d_tiles, 0, tb));
   }
   if (cfg->npix_fs > 0) {
     ctx->fs_npix = (long long)cfg->npix_fs * cfg->npix_fs;
@@ -1025,11 +1026,10 @@ p2m_status p2m_reset_maps(p2m_ctx *ctx) {
     if (ctx->d_acc64)
       CK(cudaMemsetAsync(ctx->d_acc64, 0,
                          sizeof(double) * (size_t)ctx->cfg.nmaps * (size_t)ctx->hp_npix, s));
-    if (ctx->d_lo) {
+    if (ctx->d_lo)
       CK(cudaMemsetAsync(ctx->d_lo, 0, sizeof(float) * (size_t)ctx->cfg.nmaps * (size_t)ctx->hp_npix, s));
-      CK(cudaMemsetAsync(ctx->d_tiles, 0,
-                         (size_t)((ctx->hp_npix + P2M_TILE_PIX - 1) >> P2M_TILE_SHIFT), s));
-    }
+    CK(cudaMemsetAsync(ctx->d_tiles, 0,
+                       (size_t)((ctx->hp_npix + P2M_TILE_PIX - 1) >> P2M_TILE_SHIFT), s));
     ctx->unfolded = false;
   }
   if (ctx->d_fs_acc)

@@ -16,7 +16,8 @@
  *              ring spans of a batch of halos in registers and paints their candidates
  *   scan + k_paint_full  the large halos' items, load-balanced over candidate pixels
  *   read-out   mixed precision: the maps hold the high words of a compensated sum and
- *              k_fold_lo adds the sparse low words; FP64 accumulation: k_finalize_full
+ *              k_fold_lo adds the sparse low words; FP64 and fixed-point accumulation:
+ *              k_read_tiles adds the painted tiles' sums, and k_clear_tiles clears them
  */
 #ifndef P2M_INTERNAL_H
 #define P2M_INTERNAL_H
@@ -28,7 +29,7 @@
 
 #define P2M_STREAM_CHUNK (1LL << 22) /* host records per streamed ingest chunk */
 #define P2M_BIG_RINGS 64      /* default: halos spanning more rings go through the item buffer */
-#define P2M_TILE_SHIFT 5      /* compensated path: a flagged tile is 32 pixels (128 bytes) */
+#define P2M_TILE_SHIFT 5      /* a flagged tile is 32 pixels (128 bytes of a map) */
 #define P2M_TILE_PIX (1 << P2M_TILE_SHIFT)
 #define P2M_PHITAB 4096       /* grid angles 2 pi k / P2M_PHITAB of the disc-centre phi reduction */
 
@@ -168,7 +169,8 @@ struct SweepBuffers {
   float *out[P2M_MAXMAPS];     /* float output maps */
   void *acc;                   /* full-sky FP64 accumulator (FP64-accumulating paths) */
   float *lo;                   /* compensated path: low words, map m at lo + m * npix */
-  unsigned char *tiles;        /* compensated path: 1 per tile with a nonzero low word */
+  unsigned char *tiles;        /* 1 per tile with a nonzero low word (compensated path), or that
+                                  halos may have painted (the others) */
   long long npix;
   DevCounters *ctr;
   long long *set_rec, *set_pix;
@@ -194,12 +196,14 @@ void p2m_launch_fs(const PaintParams &P, const IngestBuffers &B, long long n_max
                    int nsm);
 void p2m_launch_pair_table(float2 *dst, const float *ta, int pa, const float *tb, int pb,
                            long long nent, cudaStream_t s, int nsm);
-void p2m_launch_item_counts(const RingItem *items, long long n, unsigned int *counts,
+void p2m_launch_item_counts(const PaintParams &P, const SweepBuffers &W, unsigned int *counts,
                             cudaStream_t s, int nsm);
 void p2m_launch_paint_halos(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 void p2m_launch_paint_full(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
-void p2m_launch_finalize_full(const PaintParams &P, const void *acc, long long npix,
-                              float *const *out, int accumulate, cudaStream_t s, int nsm);
+/* read-out of the FP64 and fixed-point accumulators' flagged tiles into the maps; their clear */
+void p2m_launch_read_tiles(const PaintParams &P, const SweepBuffers &W, int add, cudaStream_t s,
+                           int nsm);
+void p2m_launch_clear_tiles(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 void p2m_launch_finalize_fs(const PaintParams &P, const void *acc, long long npix, float *out,
                             int map, double *sum, cudaStream_t s, int nsm);
 void p2m_launch_fold_lo(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);

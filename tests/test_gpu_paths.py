@@ -110,3 +110,44 @@ def ring_z(nside, ring):
     i = min(ring, 4 * nside - ring)
     z = 1 - i * i / (3.0 * nside * nside) if i < nside else (2 * nside - i) / (1.5 * nside)
     return z if ring <= 2 * nside else -z
+
+
+@pytest.mark.parametrize("cones", [0, 5])
+@pytest.mark.parametrize("nmaps", [1, 2, 3, 8])
+@pytest.mark.parametrize("nside", [1, 2, 16, 256])
+def test_painted_tiles_are_read_and_cleared(nside, nmaps, cones):
+    """The FP64 and fixed-point read-outs visit and clear only the tiles that were painted
+    (tiles may straddle the end of the map or two cones' maps): after another catalogue,
+    read or dropped by a reset, the fixed-point maps are those of a new painter bit for
+    bit, and every pixel outside them is zero."""
+    maps = tuple((0, 1 + (m & 1)) for m in range(nmaps))
+    near = catalogs.shell(81, 4000, r=(30.0, 400.0), m=(1e14, 3e15))
+    far = catalogs.shell(82, 6000, m=(1e13, 3e15))
+    tab = catalogs.table(nu=0.0)
+    off = np.linspace(0, len(near), 6).astype(np.int64), np.linspace(0, len(far), 6).astype(np.int64)
+
+    def painter():
+        pt = p2m.Painter(nside=nside, precision="fixed", maps=maps, zmax=6.0, ncones=cones,
+                         max_records=len(far))
+        pt.load_table(0, tab)
+        return pt
+
+    def paint(pt, rec, o):
+        if cones:
+            pt.paint_ensemble(rec, o)
+        else:
+            pt.paint_records(rec)
+
+    with painter() as pt:
+        paint(pt, far, off[1])
+        want = [pt.healpix(m) for m in range(nmaps)]
+    with painter() as pt:
+        for read in (True, False):
+            paint(pt, near, off[0])
+            pt.flush() if read else pt.synchronize()
+            pt.reset()
+            paint(pt, far, off[1])
+            for m in range(nmaps):
+                assert np.array_equal(pt.healpix(m), want[m])
+            pt.reset()
+            assert all(not pt.healpix(m).any() for m in range(nmaps))
