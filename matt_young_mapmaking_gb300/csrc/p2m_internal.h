@@ -168,7 +168,7 @@ struct SweepBuffers {
   long long n_items;
   float *out[P2M_MAXMAPS];     /* float output maps */
   void *acc;                   /* full-sky FP64 accumulator (FP64-accumulating paths) */
-  float *lo;                   /* compensated path: low words, map m at lo + m * npix */
+  float *lo;                   /* compensated path: low words, a pixel's nmaps side by side */
   unsigned char *tiles;        /* 1 per tile with a nonzero low word (compensated path), or that
                                   halos may have painted (the others) */
   long long npix;
