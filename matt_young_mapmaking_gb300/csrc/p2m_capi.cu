@@ -31,6 +31,7 @@ struct p2m_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   p2m_cosmo cosmo;
+  p2m_cut cut = {}; /* follows the cosmology tables and the profile tables' header */
   std::vector<float> rofz_host, zofr_host;
   float *d_rofz = nullptr, *d_zofr = nullptr;
   /* map statistics: three FP64 sums and the P(<y) bin counts */
@@ -245,6 +246,8 @@ PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
   P.ringtab = ctx->d_ringtab;
   P.ringaux = ctx->d_ringaux;
   P.phitab = ctx->d_phitab;
+  P.cut = ctx->cut;
+  if (ctx->pre.scramble || ctx->pre.centre) P.cut.fast = 0;
   P.pre = ctx->pre;
   P.pre_ord = ctx->d_pre_ord;
   P.band_u = ctx->band_u;
@@ -273,6 +276,14 @@ PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
     P.row_c = ctx->th.nrt * ctx->th.nmht;
   }
   return P;
+}
+
+/* the cuts' thresholds, after anything they depend on has changed */
+void update_cut(p2m_ctx *ctx) {
+  const PaintParams P = make_params(ctx, 7);
+  p2m_cut_thresholds(&ctx->cut, P.cut_low, P.cut_high, P.mass_fac, &ctx->cosmo,
+                     ctx->rofz_host.data(), ctx->zofr_host.data(),
+                     ctx->th_set ? ctx->th.chimaxt : 0.0f);
 }
 
 IngestBuffers ingest_buffers(const p2m_ctx *ctx, const float *records) {
@@ -781,6 +792,7 @@ p2m_status p2m_create(const p2m_config *cfg, p2m_ctx **out) {
   ctx->rofz_host.assign(P2M_NZTAB, 0.0f);
   ctx->zofr_host.assign(P2M_NZTAB, 0.0f);
   p2m_cosmo_build(&ctx->cosmo, ctx->rofz_host.data(), ctx->zofr_host.data());
+  update_cut(ctx);
   CK(cudaMalloc((void **)&ctx->d_rofz, sizeof(float) * P2M_NZTAB));
   CK(cudaMalloc((void **)&ctx->d_zofr, sizeof(float) * P2M_NZTAB));
   CK(cudaMemcpy(ctx->d_rofz, ctx->rofz_host.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice));
@@ -957,6 +969,7 @@ p2m_status p2m_set_cosmology_tables(p2m_ctx *ctx, const float *rofz, const float
   ctx->cosmo.dzofr = FDIV(zofr_rmax, (float)(n - 1));
   CK(cudaMemcpy(ctx->d_rofz, rofz, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_zofr, zofr, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice));
+  update_cut(ctx);
   return P2M_OK;
 }
 
@@ -1004,6 +1017,7 @@ p2m_status p2m_load_table(p2m_ctx *ctx, int32_t slot, const void *image, int64_t
   ctx->th = t;
   ctx->th_set = true;
   ctx->pairs_ok = false; /* the pair tables follow the tables */
+  update_cut(ctx);
   return P2M_OK;
 }
 

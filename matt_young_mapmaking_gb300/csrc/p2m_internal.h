@@ -105,6 +105,7 @@ struct PaintParams {
   int map_table[P2M_MAXMAPS], map_profile[P2M_MAXMAPS];
   int any_ksz;
   float mass_fac; /* (4./3.*mypi)*rho_0 of pks2map.f90:264 */
+  p2m_cut cut;    /* the cuts as thresholds (fast: 0 with scramble or centre) */
   p2m_cosmo cosmo;
   p2m_tabhdr th;
   int ir_c;     /* r-index and fraction for r < rmint (r = rmint + 1e-5) */

@@ -287,6 +287,84 @@ P2M_HD float p2m_ring_coord(int nside, float theta) {
   return fn * (2.0f - 1.5f * z);
 }
 
+/* ------------------------------------------------------------ cut thresholds -------- */
+
+/* The radial and mass cuts (pks2map.f90:144-160, :264, :296) and the table's chi bound
+   (maptable.f90:184,188) as comparisons of s = x^2 + y^2 + z^2 (the float sum under the root)
+   and RTH.  The float root and the float cube are monotone, so their tests against a bound
+   are tests of their argument against the first float on the other side. */
+typedef struct p2m_cut {
+  int fast;            /* the thresholds hold: use them */
+  float s_low, s_high; /* in the shell: s_low <= s <= s_high */
+  float rth_min;       /* mass cut passed: rth >= rth_min */
+  float s_keep, s_drop; /* chi bound: inside for s <= s_keep, outside for s >= s_drop, looked up
+                           in the tables between */
+} p2m_cut;
+
+static inline float p2m_next_float(float x, int up) { /* x > 0, finite */
+  uint32_t u = p2m_f2u(x);
+  return p2m_u2f(up ? u + 1u : u - 1u);
+}
+
+/* cut_low, cut_high, mass_fac: make_params'; rofz, zofr: the context's tables; chimaxt <= 0:
+   no table loaded yet (every halo is looked up) */
+static inline void p2m_cut_thresholds(p2m_cut *c, float cut_low, float cut_high, float mass_fac,
+                                      const p2m_cosmo *cosmo, const float *rofz,
+                                      const float *zofr, float chimaxt) {
+  const float fmax = 3.4028234e38f;
+  c->fast = 0;
+  c->s_keep = -1.0f;
+  c->s_drop = p2m_inff();
+  /* bounds in the range where the squares and the cube are normal floats */
+  if (!(cut_high > 1e-15f && cut_high < 1e18f && cut_low < 1e18f && mass_fac > 1e-10f &&
+        mass_fac < 1e30f))
+    return;
+  float s = FMUL(cut_high, cut_high);
+  while (FSQRT(s) > cut_high) s = p2m_next_float(s, 0);
+  while (FSQRT(p2m_next_float(s, 1)) <= cut_high) s = p2m_next_float(s, 1);
+  c->s_high = s;
+  c->s_low = 0.0f; /* s is never negative */
+  if (cut_low > 1e-15f) {
+    s = FMUL(cut_low, cut_low);
+    while (FSQRT(s) < cut_low) s = p2m_next_float(s, 1);
+    while (FSQRT(p2m_next_float(s, 0)) >= cut_low) s = p2m_next_float(s, 0);
+    c->s_low = s;
+  } else if (cut_low > 0.0f) {
+    return;
+  }
+  /* smallest rth with !(mass_fac rth^3 < 1e13): bisection over the positive floats */
+  uint32_t lo = p2m_f2u(1e-12f), hi = p2m_f2u(fmax);
+  while (hi - lo > 1u) {
+    const uint32_t mid = lo + (hi - lo) / 2u;
+    const float r = p2m_u2f(mid);
+    if (FMUL(mass_fac, FMUL(FMUL(r, r), r)) < 1e13f) lo = mid;
+    else hi = mid;
+  }
+  c->rth_min = p2m_u2f(hi);
+  c->fast = 1;
+  /* chi = rofz(zofr(chi)) against chimaxt at the nodes of zofr: with both tables rising, the
+     function rises up to its float rounding (< 1e-6), far inside the margin of 1e-5 */
+  if (!(chimaxt > 0.0f)) return;
+  float last = -p2m_inff();
+  int keep = -1, drop = -1;
+  for (int i = 0; i < P2M_NZTAB; i++) {
+    if (i > 0 && !(rofz[i] >= rofz[i - 1] && zofr[i] >= zofr[i - 1])) return;
+    const float f = p2m_lookup(rofz, cosmo->drofz, zofr[i]);
+    if (!(f >= last * (last > 0.0f ? 0.999999f : 1.000001f))) return;
+    last = f;
+    if (f <= chimaxt * 0.99999f) keep = i;
+    if (drop < 0 && f >= chimaxt * 1.00001f) drop = i;
+  }
+  if (drop >= 0 && keep > drop) return;
+  const float ck = keep > 0 ? FMUL((float)keep, cosmo->dzofr) : 0.0f;
+  if (drop < 0 && keep == P2M_NZTAB - 1) c->s_keep = p2m_inff(); /* never beyond the bound */
+  else if (keep > 0) c->s_keep = ck * ck * 0.99999f;
+  if (drop >= 0) {
+    const float cd = FMUL((float)drop, cosmo->dzofr);
+    c->s_drop = cd * cd * 1.00001f;
+  }
+}
+
 /* ------------------------------------------------- scramble and centre -------------- */
 
 /* Pre-processing of pks2map.f90:162-262 (off unless set): scramble gives every halo that
