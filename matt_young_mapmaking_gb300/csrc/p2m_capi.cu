@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstddef>
 #include <cstdlib>
@@ -65,7 +66,7 @@ struct p2m_ctx {
   long long cap_order = 0, cap_ring_key = 0;
   unsigned int *d_ring_hist = nullptr;
   long long *d_ring_off = nullptr;
-  unsigned long long *d_nbins = nullptr;
+  bool hist_dirty = false; /* it holds counts of halos that were painted without a sort */
   /* outputs: hp_npix counts every cone's pixels (ncones * cone_npix) */
   long long hp_npix = 0, fs_npix = 0;
   long long cone_npix = 0;
@@ -121,12 +122,15 @@ struct p2m_ctx {
   long long cap_counts = 0;
   long long *d_pix_off = nullptr;
   long long cap_pix_off = 0;
-  unsigned long long *d_nitems = nullptr;
   double *d_sums = nullptr; /* [0, MAXMAPS): HEALPix, [MAXMAPS, 2 MAXMAPS): flat sky */
   long long *d_set_rec = nullptr, *d_set_pix = nullptr;
   long long cap_set = 0;
   DevCounters *d_ctr = nullptr, *h_ctr = nullptr; /* h_ctr: mapped pinned host memory */
   DevCounters *h_ctr_dev = nullptr;                /* its device address */
+  volatile unsigned int *h_seq = nullptr;          /* behind it: the last ingest it stands for */
+  unsigned int *h_seq_dev = nullptr, seq = 0;
+  /* the call's own counters, and the painting's batch counter, are zero on the device */
+  bool ctr_clean = false, unit_clean = false;
   float *d_prep = nullptr;
   long long cap_prep = 0;
   std::vector<float> prep;
@@ -206,8 +210,26 @@ void join_out(p2m_ctx *ctx, cudaStream_t s) {
   cudaStreamWaitEvent(ctx->stream, ctx->ev_back, 0);
 }
 
-/* per-call counters precede the cumulative ones in DevCounters */
+/* per-call counters precede the cumulative ones in DevCounters.  A read-out leaves them
+   cleared for the next call; they are cleared here only where none came in between. */
 const size_t CALL_CTR_BYTES = offsetof(DevCounters, hp_updates);
+p2m_status clear_call_counters(p2m_ctx *ctx, cudaStream_t s) {
+  CK(cudaMemsetAsync(ctx->d_ctr, 0, CALL_CTR_BYTES, s));
+  ctx->ctr_clean = ctx->unit_clean = true;
+  return P2M_OK;
+}
+
+size_t ring_hist_bytes(const p2m_ctx *ctx) {
+  return sizeof(unsigned int) * (size_t)(4LL * ctx->cfg.nside + 1);
+}
+
+/* Up to this many halos are painted at once (a batch for every resident warp of the fused
+   kernel): they are not sorted, as an order would not change which are in flight.  Their
+   sort, of 2e4 records at Nside 256, took 22 us of a pass of 57. */
+long long unsorted_halos(const p2m_ctx *ctx) {
+  return (long long)ctx->nsm * std::min(ctx->tune.halos_grid * ctx->tune.halos_threads, 1024) /
+         32 * ctx->tune.halo_batch;
+}
 
 PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
   PaintParams P;
@@ -296,11 +318,15 @@ IngestBuffers ingest_buffers(const p2m_ctx *ctx, const float *records) {
   B.nring = ctx->d_nring;
   B.ioff = ctx->d_ioff;
   B.items = ctx->d_items_raw + ctx->n_items;
+  B.counts = ctx->d_counts + ctx->n_items;
+  B.tiles = ctx->d_lo ? nullptr : ctx->d_tiles;
   B.fs_items = ctx->d_fs_items;
   B.fs_cap = ctx->cap_fs;
   B.fs_acc = ctx->d_fs_acc;
-  B.scan_tmp = ctx->d_scan_tmp;
   B.ctr = ctx->d_ctr;
+  B.h_ctr = ctx->h_ctr_dev;
+  B.h_seq = ctx->h_seq_dev;
+  B.seq = ctx->seq;
   B.set_rec = ctx->d_set_rec;
   B.set_pix = ctx->d_set_pix;
   B.set_cap = ctx->cap_set;
@@ -374,12 +400,28 @@ p2m_status read_counters(p2m_ctx *ctx, cudaStream_t s) {
   return check_errors(ctx, s);
 }
 
-/* Everything after the per-halo set-up of one ingest call: item offsets, items, flat sky.
-   The set-up kernel has been queued on s; n_max bounds the halo count. */
-p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, long long n_max, cudaStream_t s) {
+/* waits for the counters that k_cut_setup, queued on s, hands over with sequence number
+   ctx->seq.  The host polls the number: a wait for the stream costs several us more.  Should
+   the stream end without it, its error (or the missing number) is reported. */
+p2m_status wait_counters(p2m_ctx *ctx, cudaStream_t s) {
+  for (unsigned spin = 1; *ctx->h_seq != ctx->seq; spin++) {
+    if (spin & 0xfff) continue;
+    const cudaError_t e = cudaStreamQuery(s);
+    if (e == cudaErrorNotReady) continue;
+    CK(e);
+    if (*ctx->h_seq != ctx->seq)
+      return fail(ctx, P2M_ERR_CUDA, "the cut kernel ended without its counters");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return check_errors(ctx, s);
+}
+
+/* Everything after the per-halo set-up of one ingest call: items, flat sky.  The set-up kernel
+   has been queued on s; handed: it hands its counters over (k_cut_setup). */
+p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, bool handed, cudaStream_t s) {
   IngestBuffers B = ingest_buffers(ctx, nullptr);
   /* the large halos reserved their item ranges (d_ioff, n_items) during the set-up */
-  const p2m_status err = read_counters(ctx, s);
+  const p2m_status err = handed ? wait_counters(ctx, s) : read_counters(ctx, s);
   if (err) {
     /* the call is discarded: its halos, stored past n_halos, are overwritten by the next
        call, and they leave the first-ring counts that the next sort scans */
@@ -391,9 +433,10 @@ p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, long long n_max, cuda
   long long n_halo = (long long)ctx->h_ctr->n_surv;
   long long n_items = P.nside > 0 ? (long long)ctx->h_ctr->n_items : 0;
   long long n_fs = (long long)ctx->h_ctr->n_fs_rows;
-  (void)n_max;
   CK(grow(&ctx->d_items_raw, &ctx->cap_items_raw, ctx->n_items + std::max(n_items, 1LL),
           ctx->n_items, s));
+  CK(grow(&ctx->d_counts, &ctx->cap_counts, ctx->n_items + std::max(n_items, 1LL), ctx->n_items,
+          s));
   CK(grow(&ctx->d_fs_items, &ctx->cap_fs, std::max(n_fs, 1LL)));
   B = ingest_buffers(ctx, nullptr);
   if (n_halo > 0) {
@@ -429,8 +472,16 @@ p2m_status zero_outputs(p2m_ctx *ctx, cudaStream_t s) {
   CK(cudaEventRecord(ctx->ev_zero_start, s));
   CK(cudaStreamWaitEvent(ctx->zstream, ctx->ev_zero_start, 0));
   ST(wait_reads(ctx, ctx->zstream));
-  for (int m = 0; m < ctx->cfg.nmaps; m++)
-    CK(cudaMemsetAsync(ctx->d_out[m], 0, sizeof(float) * (size_t)ctx->hp_npix, ctx->zstream));
+  /* small maps by one launch; large ones by the faster memsets */
+  bool one = ctx->cfg.nmaps > 1 && ctx->hp_npix <= (1LL << 23);
+  for (int m = 0; m < ctx->cfg.nmaps; m++) one = one && !((uintptr_t)ctx->d_out[m] & 15);
+  if (one) {
+    p2m_launch_clear_maps(ctx->d_out, ctx->cfg.nmaps, ctx->hp_npix, ctx->zstream, ctx->nsm);
+    CK(cudaGetLastError());
+  } else {
+    for (int m = 0; m < ctx->cfg.nmaps; m++)
+      CK(cudaMemsetAsync(ctx->d_out[m], 0, sizeof(float) * (size_t)ctx->hp_npix, ctx->zstream));
+  }
   CK(cudaEventRecord(ctx->ev_zero_done, ctx->zstream));
   ctx->zero_pending = true;
   ctx->outs_zeroed = true;
@@ -472,13 +523,15 @@ p2m_status begin_call(p2m_ctx *ctx, long long n, cudaStream_t s) {
       CK(cudaMalloc((void **)&ctx->d_ring_hist, sizeof(unsigned int) * (size_t)nbins));
       CK(cudaMemset(ctx->d_ring_hist, 0, sizeof(unsigned int) * (size_t)nbins));
       CK(cudaMalloc((void **)&ctx->d_ring_off, sizeof(long long) * (size_t)nbins));
-      CK(cudaMalloc((void **)&ctx->d_nbins, sizeof(unsigned long long)));
-      const unsigned long long nb = (unsigned long long)nbins;
-      CK(cudaMemcpy(ctx->d_nbins, &nb, sizeof(nb), cudaMemcpyHostToDevice));
     }
   }
+  if (ctx->hist_dirty) {
+    CK(cudaMemsetAsync(ctx->d_ring_hist, 0, ring_hist_bytes(ctx), s));
+    ctx->hist_dirty = false;
+  }
   for (int k = 0; k < P2M_NPHASE; k++) ctx->tev_used[k] = false;
-  CK(cudaMemsetAsync(ctx->d_ctr, 0, CALL_CTR_BYTES, s));
+  if (!ctx->ctr_clean) ST(clear_call_counters(ctx, s));
+  ctx->ctr_clean = false;
   return P2M_OK;
 }
 
@@ -501,7 +554,7 @@ p2m_status flush_prepared(p2m_ctx *ctx) {
   TE(PH_SETUP);
   CK(cudaStreamSynchronize(s)); /* nn and prep are host memory */
   ctx->prep.clear();
-  ST(ingest_tail(ctx, P, n, s));
+  ST(ingest_tail(ctx, P, false, s));
   ctx->rec_count += n;
   return P2M_OK;
 }
@@ -523,9 +576,7 @@ p2m_status preprocess(p2m_ctx *ctx, const float *d_rec, long long nrec, int nflo
   CK(grow(&ctx->d_pre_flags, &ctx->cap_pre_flags, nrec));
   CK(grow(&ctx->d_pre_ord, &ctx->cap_pre_ord, nrec));
   p2m_launch_pre_flags(P, d_rec, nrec, ctx->d_pre_flags, s, ctx->nsm);
-  unsigned long long nn = (unsigned long long)nrec;
-  CK(cudaMemcpyAsync(ctx->d_nitems, &nn, sizeof(nn), cudaMemcpyHostToDevice, s));
-  p2m_launch_scan_u32(ctx->d_pre_flags, ctx->d_nitems, ctx->d_pre_ord, nullptr, ctx->d_scan_tmp, s);
+  p2m_launch_scan_u32(ctx->d_pre_flags, nrec, ctx->d_pre_ord, nullptr, ctx->d_scan_tmp, s);
   for (int k = 0; k < 9; k++) ctx->centre_info[k] = 0.0f;
   if (centre) {
     CK(grow(&ctx->d_pre_last, &ctx->cap_pre_last, ntasks));
@@ -610,6 +661,7 @@ p2m_status ingest_device(p2m_ctx *ctx, const float *d_rec, long long nrec, int n
   ST(begin_call(ctx, nrec, s));
   if (pre) ST(preprocess(ctx, d_rec, nrec, nfloat, s));
   PaintParams P = make_params(ctx, nfloat);
+  ctx->seq++;
   IngestBuffers B = ingest_buffers(ctx, d_rec);
   if (ncones > 1) {
     B.cone_off = ctx->d_cone_off;
@@ -618,7 +670,8 @@ p2m_status ingest_device(p2m_ctx *ctx, const float *d_rec, long long nrec, int n
   TB(PH_CUT);
   p2m_launch_cut_setup(P, B, nrec, s, ctx->nsm);
   TE(PH_CUT);
-  p2m_status st = ingest_tail(ctx, P, nrec, s);
+  CK(cudaGetLastError());
+  p2m_status st = ingest_tail(ctx, P, true, s);
   join_out(ctx, s);
   if (st) return st;
   ctx->rec_count += nrec;
@@ -641,6 +694,11 @@ SweepBuffers sweep_buffers(const p2m_ctx *ctx) {
   W.tiles = ctx->d_tiles;
   W.npix = ctx->hp_npix;
   W.ctr = ctx->d_ctr;
+  W.h_ctr = ctx->h_ctr_dev;
+  if (ctx->hist_dirty) {
+    W.hist = ctx->d_ring_hist;
+    W.nhist = 4 * ctx->cfg.nside + 1;
+  }
   W.set_rec = ctx->d_set_rec;
   W.set_pix = ctx->d_set_pix;
   W.set_cap = ctx->cap_set;
@@ -661,29 +719,26 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   join_in(ctx, s);
   ST(wait_reads(ctx, s));
   const long long n = ctx->n_items;
-  CK(cudaMemsetAsync(ctx->d_ctr, 0, CALL_CTR_BYTES, s));
+  if (!ctx->unit_clean) ST(clear_call_counters(ctx, s));
+  ctx->ctr_clean = ctx->unit_clean = false;
   PaintParams P = make_params(ctx, 7);
   TB(PH_GROUP);
   if (n > 0) {
     /* candidate offsets of the large halos' items */
-    CK(grow(&ctx->d_counts, &ctx->cap_counts, n));
     CK(grow(&ctx->d_pix_off, &ctx->cap_pix_off, n));
-    unsigned long long nn = (unsigned long long)n;
-    CK(cudaMemcpyAsync(ctx->d_nitems, &nn, sizeof(nn), cudaMemcpyHostToDevice, s));
-    p2m_launch_item_counts(P, sweep_buffers(ctx), ctx->d_counts, s, ctx->nsm);
-    p2m_launch_scan_u32(ctx->d_counts, ctx->d_nitems, ctx->d_pix_off, &ctx->d_ctr->n_pix,
-                        ctx->d_scan_tmp, s);
+    p2m_launch_scan_u32(ctx->d_counts, n, ctx->d_pix_off, &ctx->d_ctr->n_pix, ctx->d_scan_tmp, s);
   }
   SweepBuffers W = sweep_buffers(ctx);
-  if (ctx->tune.sort_halos && ctx->d_ring_hist) {
+  if (ctx->tune.sort_halos && ctx->d_ring_hist && ctx->n_halos <= unsorted_halos(ctx)) {
+    ctx->hist_dirty = true;
+  } else if (ctx->tune.sort_halos && ctx->d_ring_hist) {
     /* counting sort of the halos by first ring (keys and counts came from the set-up):
        the halos painted at any one time then cover a narrow band of rings, a contiguous
        stretch of each map that the L2 holds */
     const long long nbins = 4LL * ctx->cfg.nside + 1;
     CK(grow(&ctx->d_order, &ctx->cap_order, std::max(ctx->n_halos, 1LL)));
-    p2m_launch_scan_u32(ctx->d_ring_hist, ctx->d_nbins, ctx->d_ring_off, nullptr, ctx->d_scan_tmp, s);
+    p2m_launch_ring_scan(ctx->d_ring_hist, (int)nbins, ctx->d_ring_off, s);
     p2m_launch_ring_scatter(ctx->d_ring_key, ctx->n_halos, ctx->d_ring_off, ctx->d_order, s, ctx->nsm);
-    CK(cudaMemsetAsync(ctx->d_ring_hist, 0, sizeof(unsigned int) * (size_t)nbins, s));
     W.order = ctx->d_order;
   }
   TE(PH_GROUP);
@@ -741,12 +796,13 @@ p2m_status sweep(p2m_ctx *ctx, cudaStream_t s) {
   }
   TE(PH_READOUT);
   CK(cudaGetLastError());
-  /* the counters go to mapped host memory without a wait.  A device error flag raised
-     by the painting is reported by the next call that waits for the device: the next
-     ingest, a host read-out, the statistics or p2m_synchronize.  The fold and the FP64
-     read-out leave the accumulators clear either way. */
-  p2m_launch_copy_counters(ctx->d_ctr, ctx->h_ctr_dev, s);
-  CK(cudaGetLastError());
+  /* the read-out also copies the counters to mapped host memory, without a wait, and clears
+     the call's own.  A device error flag raised by the painting is reported by the next call
+     that waits for the device: the next ingest, a host read-out, the statistics or
+     p2m_synchronize.  The fold and the FP64 read-out leave the accumulators clear either
+     way. */
+  ctx->ctr_clean = ctx->unit_clean = true;
+  ctx->hist_dirty = false;
   join_out(ctx, s);
   ctx->unfolded = false;
   ctx->swept = true;
@@ -865,12 +921,15 @@ p2m_status p2m_create(const p2m_config *cfg, p2m_ctx **out) {
     CK(cudaMalloc((void **)&ctx->d_fs_out, sizeof(float) * (size_t)ctx->fs_npix));
   }
   CK(cudaMalloc((void **)&ctx->d_scan_tmp, sizeof(long long) * 1024));
-  CK(cudaMalloc((void **)&ctx->d_ctr, sizeof(DevCounters)));
-  CK(cudaHostAlloc((void **)&ctx->h_ctr, sizeof(DevCounters), cudaHostAllocMapped));
+  /* the map sums lie behind the counters: a reset clears both at once */
+  CK(cudaMalloc((void **)&ctx->d_ctr, sizeof(DevCounters) + sizeof(double) * 2 * P2M_MAXMAPS));
+  ctx->d_sums = (double *)(ctx->d_ctr + 1);
+  CK(cudaHostAlloc((void **)&ctx->h_ctr, sizeof(DevCounters) + sizeof(unsigned int), cudaHostAllocMapped));
+  memset(ctx->h_ctr, 0, sizeof(DevCounters) + sizeof(unsigned int));
   CK(cudaHostGetDevicePointer((void **)&ctx->h_ctr_dev, ctx->h_ctr, 0));
-  CK(cudaMalloc((void **)&ctx->d_nitems, sizeof(unsigned long long)));
+  ctx->h_seq = (volatile unsigned int *)(ctx->h_ctr + 1);
+  ctx->h_seq_dev = (unsigned int *)(ctx->h_ctr_dev + 1);
   CK(cudaMalloc((void **)&ctx->d_pre_bits, sizeof(unsigned int)));
-  CK(cudaMalloc((void **)&ctx->d_sums, sizeof(double) * 2 * P2M_MAXMAPS));
   if (cfg->flags & P2M_FLAG_RECORD_SETS) {
     /* (record, pixel) pairs kept; P2M_SET_CAP raises it for catalogues whose discs hold
        more pixels in all (16 bytes of device memory per pair) */
@@ -896,11 +955,11 @@ void p2m_destroy(p2m_ctx *ctx) {
   void *ptrs[] = {ctx->d_rofz, ctx->d_zofr, ctx->d_ringtab, ctx->d_ringaux, ctx->d_phitab, ctx->d_acc64, ctx->d_fs_acc,
                   ctx->d_fs_out, ctx->d_halos, ctx->d_items_raw,
                   ctx->d_nring, ctx->d_ioff, ctx->d_fs_items, ctx->d_scan_tmp, ctx->d_counts,
-                  ctx->d_pix_off, ctx->d_nitems, ctx->d_sums, ctx->d_set_rec, ctx->d_set_pix,
+                  ctx->d_pix_off, ctx->d_set_rec, ctx->d_set_pix,
                   ctx->d_ctr, ctx->d_prep, ctx->d_lo, ctx->d_tiles,
                   ctx->d_pre_flags, ctx->d_pre_bits, ctx->d_pre_ord, ctx->d_pre_last,
                   ctx->d_cone_off, ctx->d_stage[0], ctx->d_stage[1], ctx->d_order,
-                  ctx->d_ring_key, ctx->d_ring_hist, ctx->d_ring_off, ctx->d_nbins,
+                  ctx->d_ring_key, ctx->d_ring_hist, ctx->d_ring_off,
                   ctx->d_mstat, ctx->d_hist, ctx->d_fits[0], ctx->d_fits[1]};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -1025,6 +1084,7 @@ p2m_status p2m_reset_maps(p2m_ctx *ctx) {
   if (!ctx) return P2M_ERR_BADARG;
   CK(cudaSetDevice(ctx->cfg.device));
   cudaStream_t s = ctx->stream;
+  const bool dropped = ctx->n_halos > 0; /* ingested and never painted */
   ctx->prep.clear();
   ctx->n_halos = 0;
   ctx->n_items = 0;
@@ -1048,10 +1108,11 @@ p2m_status p2m_reset_maps(p2m_ctx *ctx) {
   }
   if (ctx->d_fs_acc)
     CK(cudaMemsetAsync(ctx->d_fs_acc, 0, 8 * (size_t)ctx->cfg.nmaps * (size_t)ctx->fs_npix, s));
-  if (ctx->d_ring_hist)
-    CK(cudaMemsetAsync(ctx->d_ring_hist, 0, sizeof(unsigned int) * (size_t)(4LL * ctx->cfg.nside + 1), s));
-  CK(cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), s));
-  CK(cudaMemsetAsync(ctx->d_sums, 0, sizeof(double) * 2 * P2M_MAXMAPS, s));
+  if (ctx->d_ring_hist && (dropped || ctx->hist_dirty))
+    CK(cudaMemsetAsync(ctx->d_ring_hist, 0, ring_hist_bytes(ctx), s));
+  ctx->hist_dirty = false;
+  CK(cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters) + sizeof(double) * 2 * P2M_MAXMAPS, s));
+  ctx->ctr_clean = ctx->unit_clean = true;
   return P2M_OK;
 }
 

@@ -7,9 +7,8 @@
  *              value is not identically zero, queued in shared memory, and per queued
  *              halo the loop quantities of pks2map.f90:284-298, disc radius and centre,
  *              interpolation constants, candidate ring range, flat-sky box
- *   scan       rings of the large halos (more than big_rings rings) -> item offsets
- *   k_items    per (large halo, ring) item: FP32 superset of the ring's pixel span and
- *              the ring constants of the disc test
+ *   k_items    per (large halo, ring) item (more than big_rings rings): FP32 superset of the
+ *              ring's pixel span and the ring constants of the disc test
  *   k_paint_fs flat-sky rows (exact float sequence of the reference)
  * Sweep:
  *   k_paint_halos  the other halos, enumeration fused with painting: a warp builds the
@@ -43,6 +42,7 @@ struct DevCounters {
   unsigned long long val_checked, val_bad_set, val_bad_index;
   unsigned int val_max_du; /* float bits of the largest |u_fast - u_exact| */
   unsigned int err;        /* P2M_DEVERR_* raised since it was last reported */
+  unsigned int done, pad1; /* blocks of k_cut_setup that are done (zero between launches) */
 };
 
 enum {
@@ -151,11 +151,17 @@ struct IngestBuffers {
   unsigned int *nring;  /* rings per large halo, 0 for the others */
   long long *ioff;      /* item offset per halo (call-local) */
   RingItem *items;      /* items of this call */
+  unsigned int *counts; /* candidates of each item */
+  unsigned char *tiles; /* FP64 and fixed-point accumulation: the maps' tile flags, else null */
   FsItem *fs_items;
   long long fs_cap;
   void *fs_acc;
-  long long *scan_tmp;
   DevCounters *ctr;
+  /* mapped host memory: the last block of k_cut_setup copies the counters there and then
+     stores seq, which the host waits for */
+  DevCounters *h_ctr;
+  unsigned int *h_seq;
+  unsigned int seq;
   long long *set_rec, *set_pix;
   long long set_cap;
 };
@@ -174,6 +180,9 @@ struct SweepBuffers {
                                   halos may have painted (the others) */
   long long npix;
   DevCounters *ctr;
+  DevCounters *h_ctr; /* mapped host copy, written by the read-out */
+  unsigned int *hist; /* first-ring counts that the read-out clears, or null */
+  int nhist;
   long long *set_rec, *set_pix;
   long long set_cap;
   const int *order;            /* halos in painting order (sorted by first ring), or null */
@@ -189,16 +198,19 @@ void p2m_launch_pre_centre(const PaintParams &P, const float *records, long long
                            long long *last, cudaStream_t s, int nsm);
 void p2m_launch_setup_prepared(const PaintParams &P, const IngestBuffers &B, const float *prep,
                                long long n, cudaStream_t s, int nsm);
-void p2m_launch_scan_u32(const unsigned int *in, const unsigned long long *n_ptr, long long *out,
+/* exclusive prefix sums of n counts; *total (if not null) their sum */
+void p2m_launch_scan_u32(const unsigned int *in, long long n, long long *out,
                          unsigned long long *total, long long *tmp, cudaStream_t s);
+/* exclusive prefix sums of the nbins first-ring counts, which are cleared */
+void p2m_launch_ring_scan(unsigned int *hist, int nbins, long long *off, cudaStream_t s);
+/* zeroes the maps of n floats (n a multiple of 4) with one launch */
+void p2m_launch_clear_maps(float *const *maps, int nmaps, long long n, cudaStream_t s, int nsm);
 void p2m_launch_items(const PaintParams &P, const IngestBuffers &B, long long n_max,
                       cudaStream_t s, int nsm);
 void p2m_launch_fs(const PaintParams &P, const IngestBuffers &B, long long n_max, cudaStream_t s,
                    int nsm);
 void p2m_launch_pair_table(float2 *dst, const float *ta, int pa, const float *tb, int pb,
                            long long nent, cudaStream_t s, int nsm);
-void p2m_launch_item_counts(const PaintParams &P, const SweepBuffers &W, unsigned int *counts,
-                            cudaStream_t s, int nsm);
 void p2m_launch_paint_halos(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 void p2m_launch_paint_full(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 /* read-out of the FP64 and fixed-point accumulators' flagged tiles into the maps; their clear */
