@@ -1774,6 +1774,7 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   K.nu = nu;
   K.alpha = alpha_cmb;
   K.model = model;
+  K.neg_zero = -0.0f;
   PaintParams P;
   memset(&P, 0, sizeof(P));
   P.cosmo = cosmo;

@@ -242,6 +242,7 @@ void p2m_launch_ring_unhist(const int *keys, long long n, unsigned int *hist, cu
 struct TableConsts {
   float y0, tau0, x0const, nu, alpha;
   int model;
+  float neg_zero; /* -0: see mul2_sep */
 };
 void p2m_launch_maptable(const PaintParams &P, const TableConsts &K, const p2m_tabhdr &th,
                          float *d_table, cudaStream_t s);
