@@ -151,3 +151,38 @@ def test_painted_tiles_are_read_and_cleared(nside, nmaps, cones):
                 assert np.array_equal(pt.healpix(m), want[m])
             pt.reset()
             assert all(not pt.healpix(m).any() for m in range(nmaps))
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+@pytest.mark.parametrize("nside", [1, 2, 64, 512])
+def test_map_statistics_of_any_alignment(nside, offset):
+    """Moments and P(<y) of maps read 16 bytes at a time or one value at a time (a bound
+    buffer off its 16-byte alignment), and of flat-sky maps whose size is no multiple of
+    4.  Sums: float-float per thread (2^-44) and FP64 across threads, 1e-12 of the sum of
+    magnitudes; counts: equal."""
+    import torch
+    rec = np.concatenate([catalogs.shell(91, 20_000, m=(1e13, 3e15)),
+                          catalogs.cone(92, 500, (0, 0, 1), 3.0)])
+    npix = 12 * nside * nside
+    buf = torch.full((npix + 4,), 7.0, dtype=torch.float32, device="cuda")
+    with p2m.Painter(nside=nside, npix_fs=63, fov_deg=10.0, zmax=6.0, max_records=len(rec)) as pt:
+        pt.load_table(0, catalogs.table(nu=0.0))
+        pt.bind_healpix_device(0, buf[offset:].data_ptr())
+        pt.paint_records(rec)
+        mom, rms, dpdy = pt.map_stats(0)
+        fmom, frms, _ = pt.map_stats(0, flatsky=True)
+        flat = pt.flatsky(0)
+        hp = pt.healpix(0)
+    assert np.array_equal(hp, buf[offset:offset + npix].cpu().numpy())
+    assert (buf[:offset] == 7.0).all() and (buf[offset + npix:] == 7.0).all()
+    for x, m, r in ((hp, mom, rms), (flat, fmom, frms)):
+        x = x.astype(np.float64)
+        for k in range(3):
+            assert abs(m[k] - (x ** (k + 1)).mean()) <= 1e-12 * (np.abs(x) ** (k + 1)).mean()
+        var = ((x - x.mean()) ** 2).mean()
+        assert abs(r * r - var) <= 1e-11 * (x * x).mean()
+    dy = np.float32(1e-4) / np.float32(10000)
+    q = hp / dy
+    m = q[(q > -1) & (q < 10000)].astype(np.int64)
+    count = np.bincount(m, minlength=10000).astype(np.float32)
+    assert np.array_equal(dpdy, np.cumsum(count / np.float32(npix), dtype=np.float32))
