@@ -1778,15 +1778,25 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   PaintParams P;
   memset(&P, 0, sizeof(P));
   P.cosmo = cosmo;
-  float *d_rofz = nullptr, *d_zofr = nullptr, *d_tab = nullptr;
-  CK(cudaMalloc((void **)&d_rofz, sizeof(float) * P2M_NZTAB));
-  CK(cudaMalloc((void **)&d_zofr, sizeof(float) * P2M_NZTAB));
-  CK(cudaMalloc((void **)&d_tab, sizeof(float) * (size_t)th.nelem));
-  CK(cudaMemcpy(d_rofz, rofz.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d_zofr, zofr.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice));
+  /* scratch of this call, on a stream of its own */
+  struct Scratch {
+    cudaStream_t s = nullptr;
+    void *p[3] = {nullptr, nullptr, nullptr};
+    ~Scratch() {
+      for (void *q : p) p2m_pool_free(q, s);
+      if (s) cudaStreamDestroy(s);
+    }
+  } sc;
+  CK(cudaStreamCreateWithFlags(&sc.s, cudaStreamNonBlocking));
+  CK(p2m_pool_alloc(&sc.p[0], sizeof(float) * P2M_NZTAB, sc.s));
+  CK(p2m_pool_alloc(&sc.p[1], sizeof(float) * P2M_NZTAB, sc.s));
+  CK(p2m_pool_alloc(&sc.p[2], sizeof(float) * (size_t)th.nelem, sc.s));
+  float *d_rofz = (float *)sc.p[0], *d_zofr = (float *)sc.p[1], *d_tab = (float *)sc.p[2];
+  CK(cudaMemcpyAsync(d_rofz, rofz.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice, sc.s));
+  CK(cudaMemcpyAsync(d_zofr, zofr.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice, sc.s));
   P.rofz = d_rofz;
   P.zofr = d_zofr;
-  p2m_launch_maptable(P, K, th, d_tab, 0);
+  p2m_launch_maptable(P, K, th, d_tab, sc.s);
   CK(cudaGetLastError());
   char *b = (char *)image;
   memcpy(b + 0, &th.nchit, 4);
@@ -1798,10 +1808,8 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   memcpy(b + 24, &th.mhmaxt, 4);
   memcpy(b + 28, &th.rmint, 4);
   memcpy(b + 32, &th.rmaxt, 4);
-  CK(cudaMemcpy(b + 36, d_tab, sizeof(float) * (size_t)th.nelem, cudaMemcpyDeviceToHost));
-  cudaFree(d_rofz);
-  cudaFree(d_zofr);
-  cudaFree(d_tab);
+  CK(cudaMemcpyAsync(b + 36, d_tab, sizeof(float) * (size_t)th.nelem, cudaMemcpyDeviceToHost, sc.s));
+  CK(cudaStreamSynchronize(sc.s));
   return P2M_OK;
 }
 

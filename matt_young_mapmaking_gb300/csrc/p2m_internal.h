@@ -239,6 +239,13 @@ void p2m_launch_ring_scatter(const int *keys, long long n, long long *off, int *
 /* takes halos [0, n) of a discarded ingest back out of the first-ring counts */
 void p2m_launch_ring_unhist(const int *keys, long long n, unsigned int *hist, cudaStream_t s,
                             int nsm);
+/* Stream-ordered device memory for the calls that need scratch for their own duration only (the
+   spectra, the table maker), from a pool of the current device that keeps up to 256 MB between
+   calls (any thread's and stream's) and returns the rest when a stream is waited for: making
+   and dropping such buffers took half of a 1024^2 flat-sky call.  Free on the same stream. */
+cudaError_t p2m_pool_alloc(void **out, size_t bytes, cudaStream_t s);
+void p2m_pool_free(void *p, cudaStream_t s);
+
 struct TableConsts {
   float y0, tau0, x0const, nu, alpha;
   int model;

@@ -55,6 +55,46 @@
 
 #include "../../include/p2m.h"
 #include "../../include/p2m_tools.h"
+#include "p2m_internal.h"
+
+#include <mutex>
+
+namespace {
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pools[64] = {};
+}  // namespace
+
+cudaError_t p2m_pool_alloc(void **out, size_t bytes, cudaStream_t s) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pools[dev]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t made;
+      e = cudaMemPoolCreate(&made, &props);
+      if (e != cudaSuccess) return e;
+      unsigned long long keep = 256ull << 20;
+      e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) {
+        cudaMemPoolDestroy(made);
+        return e;
+      }
+      g_pools[dev] = made;
+    }
+    pool = g_pools[dev];
+  }
+  return cudaMallocFromPoolAsync(out, bytes ? bytes : 1, pool, s);
+}
+void p2m_pool_free(void *p, cudaStream_t s) {
+  if (p) cudaFreeAsync(p, s);
+}
 
 namespace {
 
@@ -69,7 +109,7 @@ constexpr int ALM_GROUP = ALM_THREADS * ALM_RINGS;
 constexpr int ALM_LC = 64; /* values of l between rescalings */
 constexpr int ALM_LB = 8;  /* values of l summed before a warp reduces them together */
 constexpr int ALM_WARPS = ALM_THREADS / 32;
-constexpr int FFT_THREADS = 512;
+constexpr int FFT_THREADS = 256;
 constexpr int FFT_MAX_POW2 = 8192;
 constexpr int DFT_MAX = 2048;
 
@@ -135,17 +175,56 @@ __host__ __device__ __forceinline__ int conv_len(int n) {
   return l;
 }
 
-/* In-place radix-2 FFT of the len complex values in shared memory (len a power of two) by the
-   whole block, input in bit-reversed order.  tw[k] = exp(-2 pi i k / twlen), twlen >= len. */
+/* u + w v and u - w v in six FP64 operations: u - w v as 2 u - (u + w v) */
+__device__ __forceinline__ void butterfly(double2 &u, double2 &v, double2 w) {
+  const double ar = fma(-v.y, w.y, fma(v.x, w.x, u.x)), ai = fma(v.y, w.x, fma(v.x, w.y, u.y));
+  v = make_double2(fma(2.0, u.x, -ar), fma(2.0, u.y, -ai));
+  u = make_double2(ar, ai);
+}
+__device__ __forceinline__ void butterfly1(double2 &u, double2 &v) { /* w = 1 */
+  const double2 a = make_double2(u.x + v.x, u.y + v.y);
+  v = make_double2(u.x - v.x, u.y - v.y);
+  u = a;
+}
+
+/* In-place FFT of the len complex values in shared memory (len a power of two) by the whole
+   block, input in bit-reversed order.  tw[k] = exp(-2 pi i k / twlen), twlen >= len.  Two
+   radix-2 stages per pass (after one alone where their number is odd): a thread takes four
+   values through both in registers, half the passes over shared memory and half the
+   barriers.  FP64 issue bounds it: 6 operations a butterfly, 4 in the first two stages,
+   whose factors are 1 and -i. */
 __device__ void block_fft(double2 *sz, int len, const double2 *__restrict__ tw, int twlen) {
-  for (int half = 1; half < len; half <<= 1) {
-    const int stride = twlen / (2 * half);
-    for (int b = threadIdx.x; b < len / 2; b += blockDim.x) {
+  int half = 1;
+  if ((31 - __clz(len)) & 1) {
+    for (int b = threadIdx.x; b < len / 2; b += blockDim.x) butterfly1(sz[2 * b], sz[2 * b + 1]);
+    half = 2;
+    __syncthreads();
+  }
+  for (; half < len; half <<= 2) {
+    /* stages half and 2 half: values i, i + half, i + 2 half, i + 3 half */
+    const int s1 = twlen / (2 * half), s2 = s1 >> 1;
+    for (int b = threadIdx.x; b < len / 4; b += blockDim.x) {
       const int pos = b & (half - 1);
-      const int i0 = ((b - pos) << 1) + pos, i1 = i0 + half;
-      const double2 u = sz[i0], t = cmul(sz[i1], tw[pos * stride]);
-      sz[i0] = make_double2(u.x + t.x, u.y + t.y);
-      sz[i1] = make_double2(u.x - t.x, u.y - t.y);
+      double2 *z = sz + (((b - pos) << 2) + pos);
+      double2 a0 = z[0], a1 = z[half], a2 = z[2 * half], a3 = z[3 * half];
+      if (half == 1) {
+        butterfly1(a0, a1);
+        butterfly1(a2, a3);
+        butterfly1(a0, a2);
+        const double2 r = make_double2(a3.y, -a3.x); /* -i a3 */
+        a3 = r;
+        butterfly1(a1, a3);
+      } else {
+        const double2 w1 = tw[pos * s1], w2 = tw[pos * s2];
+        butterfly(a0, a1, w1);
+        butterfly(a2, a3, w1);
+        butterfly(a0, a2, w2);
+        butterfly(a1, a3, make_double2(w2.y, -w2.x)); /* -i w2 */
+      }
+      z[0] = a0;
+      z[half] = a1;
+      z[2 * half] = a2;
+      z[3 * half] = a3;
     }
     __syncthreads();
   }
@@ -568,26 +647,19 @@ __global__ void k_twiddles(double2 *tw, int n) {
   tw[k] = make_double2(c, -s);
 }
 
-/* in-place radix-2 FFT of each row (n a power of two, n >= 4), one block per row */
+/* in-place FFT of each row (n a power of two, n >= 4), one block per row; FIRST: the rows are
+   made from the maps (a + i b) */
+template <int FIRST>
 __global__ void __launch_bounds__(FFT_THREADS)
-    k_fft_rows(double2 *__restrict__ z, int n, int logn, const double2 *__restrict__ tw) {
+    k_fft_rows(double2 *__restrict__ z, const float *__restrict__ a, const float *__restrict__ b,
+               int n, int logn, const double2 *__restrict__ tw) {
   extern __shared__ double2 sz[];
-  double2 *row = z + (size_t)blockIdx.x * n;
-  for (int j = threadIdx.x; j < n; j += FFT_THREADS) sz[__brev((unsigned)j) >> (32 - logn)] = row[j];
+  const size_t at = (size_t)blockIdx.x * n;
+  for (int j = threadIdx.x; j < n; j += FFT_THREADS)
+    sz[bitrev(j, logn)] = FIRST ? make_double2((double)a[at + j], b ? (double)b[at + j] : 0.0) : z[at + j];
   __syncthreads();
-  for (int half = 1; half < n; half <<= 1) {
-    const int stride = n / (2 * half);
-    for (int b = threadIdx.x; b < n / 2; b += FFT_THREADS) {
-      const int pos = b & (half - 1);
-      const int i0 = ((b - pos) << 1) + pos, i1 = i0 + half;
-      const double2 w = tw[pos * stride], u = sz[i0], v = sz[i1];
-      const double vr = v.x * w.x - v.y * w.y, vi = v.x * w.y + v.y * w.x;
-      sz[i0] = make_double2(u.x + vr, u.y + vi);
-      sz[i1] = make_double2(u.x - vr, u.y - vi);
-    }
-    __syncthreads();
-  }
-  for (int j = threadIdx.x; j < n; j += FFT_THREADS) row[j] = sz[j];
+  block_fft(sz, n, tw, n);
+  for (int j = threadIdx.x; j < n; j += FFT_THREADS) z[at + j] = sz[j];
 }
 
 /* direct DFT of each row into out (any n <= DFT_MAX), one block per row */
@@ -633,46 +705,67 @@ __global__ void k_transpose(const double2 *__restrict__ in, double2 *__restrict_
   }
 }
 
-/* per bin: modes, sum ell, |F_a|^2, Re F_a conj F_b, |F_b|^2 over |k1|, |k2| <= kmax */
-__global__ void k_fs_bins(const double2 *__restrict__ z, int n, double ell_fund, double ell_max,
-                          int nbins, int kmax, double *__restrict__ acc) {
+/* Per bin: modes, sum ell, |F_a|^2, Re F_a conj F_b, |F_b|^2 over |k1|, |k2| <= kmax.  The maps
+   are real, so k and -k contribute alike: only k1 > 0, or k1 = 0 with k2 > 0, is visited and
+   counted twice.  A thread takes a run of consecutive k2 and adds to the block's bins in shared
+   memory when its bin changes. */
+#define FS_RUN 4
+__global__ void __launch_bounds__(256)
+    k_fs_bins(const double2 *__restrict__ z, int n, double ell_fund, double ell_max, int nbins,
+              int kmax, double *__restrict__ acc) {
   extern __shared__ double sb[];
   for (int i = threadIdx.x; i < nbins * 5; i += blockDim.x) sb[i] = 0.0;
   __syncthreads();
-  const long long side = 2LL * kmax + 1, total = side * side;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int k1 = (int)(idx / side) - kmax, k2 = (int)(idx % side) - kmax;
-    if (k1 == 0 && k2 == 0) continue;
-    const double ell = ell_fund * sqrt((double)k1 * k1 + (double)k2 * k2);
-    if (ell > ell_max) continue;
-    const int b = min((int)(ell / ell_max * nbins), nbins - 1);
-    const int i1 = (k1 + n) % n, i2 = (k2 + n) % n, j1 = (n - k1) % n, j2 = (n - k2) % n;
-    const double2 zk = z[(size_t)i1 * n + i2], zm = z[(size_t)j1 * n + j2];
-    /* F_a = (Z(k) + conj Z(-k)) / 2, F_b = (Z(k) - conj Z(-k)) / 2i */
-    const double far = 0.5 * (zk.x + zm.x), fai = 0.5 * (zk.y - zm.y);
-    const double fbr = 0.5 * (zk.y + zm.y), fbi = -0.5 * (zk.x - zm.x);
-    atomicAdd(&sb[b * 5 + 0], 1.0);
-    atomicAdd(&sb[b * 5 + 1], ell);
-    atomicAdd(&sb[b * 5 + 2], far * far + fai * fai);
-    atomicAdd(&sb[b * 5 + 3], far * fbr + fai * fbi);
-    atomicAdd(&sb[b * 5 + 4], fbr * fbr + fbi * fbi);
+  const int side = 2 * kmax + 1, runs = (side + FS_RUN - 1) / FS_RUN;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < (kmax + 1) * runs;
+       idx += gridDim.x * blockDim.x) {
+    const int k1 = idx / runs, first = (idx - k1 * runs) * FS_RUN - kmax;
+    const int last = min(first + FS_RUN - 1, kmax);
+    const int i1 = k1, j1 = k1 ? n - k1 : 0;
+    int bin = -1;
+    double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int k2 = k1 ? first : max(first, 1); k2 <= last; k2++) {
+      const double ell = ell_fund * sqrt((double)k1 * k1 + (double)k2 * k2);
+      if (ell > ell_max) continue;
+      const int b = min((int)(ell / ell_max * nbins), nbins - 1);
+      if (b != bin && bin >= 0) {
+        for (int c = 0; c < 5; c++) {
+          atomicAdd(&sb[bin * 5 + c], 2.0 * s[c]);
+          s[c] = 0.0;
+        }
+      }
+      bin = b;
+      const int i2 = k2 < 0 ? k2 + n : k2, j2 = k2 > 0 ? n - k2 : -k2;
+      const double2 zk = z[(size_t)i1 * n + i2], zm = z[(size_t)j1 * n + j2];
+      /* F_a = (Z(k) + conj Z(-k)) / 2, F_b = (Z(k) - conj Z(-k)) / 2i */
+      const double far = 0.5 * (zk.x + zm.x), fai = 0.5 * (zk.y - zm.y);
+      const double fbr = 0.5 * (zk.y + zm.y), fbi = -0.5 * (zk.x - zm.x);
+      s[0] += 1.0;
+      s[1] += ell;
+      s[2] += far * far + fai * fai;
+      s[3] += far * fbr + fai * fbi;
+      s[4] += fbr * fbr + fbi * fbi;
+    }
+    if (bin >= 0)
+      for (int c = 0; c < 5; c++) atomicAdd(&sb[bin * 5 + c], 2.0 * s[c]);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nbins * 5; i += blockDim.x)
     if (sb[i] != 0.0) atomicAdd(&acc[i], sb[i]);
 }
 
-/* device buffers released on every return path */
+/* device buffers of one call, used on its stream only and released on every return path */
 struct DevBufs {
+  cudaStream_t s;
   std::vector<void *> p;
+  explicit DevBufs(cudaStream_t stream) : s(stream) {}
   ~DevBufs() {
-    for (void *q : p) cudaFree(q);
+    for (void *q : p) p2m_pool_free(q, s);
   }
   template <class T>
   cudaError_t get(T **out, size_t bytes) {
     void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, bytes ? bytes : 1);
+    cudaError_t e = p2m_pool_alloc(&q, bytes, s);
     if (e == cudaSuccess) p.push_back(q);
     *out = (T *)q;
     return e;
@@ -728,7 +821,7 @@ int32_t p2m_cl_healpix(int32_t device, const float *map_a, const float *map_b, i
   if (!scope.ok) return P2M_ERR_CUDA;
   Stream st;
   if (!st.s) return P2M_ERR_CUDA;
-  DevBufs B;
+  DevBufs B(st.s);
   const long long npix = 12LL * nside * nside;
   const int nrings = 2 * nside;
   const size_t nalm = alm_row(lmax + 1, lmax); /* (lmax + 1)(lmax + 2) / 2 */
@@ -834,7 +927,7 @@ int32_t p2m_cl_flatsky(int32_t device, const float *map_a, const float *map_b, i
   if (!scope.ok) return P2M_ERR_CUDA;
   Stream st;
   if (!st.s) return P2M_ERR_CUDA;
-  DevBufs B;
+  DevBufs B(st.s);
   const long long n2 = (long long)npix * npix;
   float *d_a = nullptr, *d_b = nullptr;
   double2 *z = nullptr, *z2 = nullptr, *tw = nullptr;
@@ -849,19 +942,19 @@ int32_t p2m_cl_flatsky(int32_t device, const float *map_a, const float *map_b, i
   if (map_b)
     SP_CK(cudaMemcpyAsync(d_b, map_b, sizeof(float) * (size_t)n2, cudaMemcpyHostToDevice, st.s));
   SP_CK(cudaMemsetAsync(d_acc, 0, sizeof(double) * 5 * (size_t)nbins, st.s));
-  k_fs_pack<<<(int)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, st.s>>>(d_a, d_b, n2, z);
-  SP_CK(cudaGetLastError());
   const dim3 tb(32, 8), tg((npix + 31) / 32, (npix + 31) / 32);
   if (pow2) {
     const int logn = ilog2(npix);
     const size_t smem = sizeof(double2) * (size_t)npix;
-    SP_CK(cudaFuncSetAttribute(k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SP_CK(cudaFuncSetAttribute(k_fft_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SP_CK(cudaFuncSetAttribute(k_fft_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_twiddles<<<(npix / 2 + 255) / 256, 256, 0, st.s>>>(tw, npix);
-    k_fft_rows<<<npix, FFT_THREADS, smem, st.s>>>(z, npix, logn, tw);
+    k_fft_rows<1><<<npix, FFT_THREADS, smem, st.s>>>(z, d_a, d_b, npix, logn, tw);
     k_transpose<<<tg, tb, 0, st.s>>>(z, z2, npix);
-    k_fft_rows<<<npix, FFT_THREADS, smem, st.s>>>(z2, npix, logn, tw);
+    k_fft_rows<0><<<npix, FFT_THREADS, smem, st.s>>>(z2, nullptr, nullptr, npix, logn, tw);
   } else {
     const size_t smem = sizeof(double2) * (size_t)npix;
+    k_fs_pack<<<(int)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, st.s>>>(d_a, d_b, n2, z);
     k_dft_rows<<<npix, 256, smem, st.s>>>(z, z2, npix);
     k_transpose<<<tg, tb, 0, st.s>>>(z2, z, npix);
     k_dft_rows<<<npix, 256, smem, st.s>>>(z, z2, npix);
@@ -871,7 +964,7 @@ int32_t p2m_cl_flatsky(int32_t device, const float *map_a, const float *map_b, i
   int kmax = (int)std::ceil(ell_max / ell_fund);
   kmax = std::min(kmax, npix / 2 - 1); /* the Nyquist line is left out */
   if (kmax >= 1) {
-    const long long total = (2LL * kmax + 1) * (2LL * kmax + 1);
+    const long long total = (kmax + 1LL) * ((2LL * kmax + FS_RUN) / FS_RUN);
     const int grid = (int)std::min<long long>((total + 255) / 256, 1024);
     k_fs_bins<<<grid, 256, sizeof(double) * 5 * (size_t)nbins, st.s>>>(
         z2, npix, ell_fund, ell_max, nbins, kmax, d_acc);

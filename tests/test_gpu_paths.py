@@ -186,3 +186,24 @@ def test_map_statistics_of_any_alignment(nside, offset):
     m = q[(q > -1) & (q < 10000)].astype(np.int64)
     count = np.bincount(m, minlength=10000).astype(np.float32)
     assert np.array_equal(dpdy, np.cumsum(count / np.float32(npix), dtype=np.float32))
+
+
+@pytest.mark.parametrize("two", [True, False])
+@pytest.mark.parametrize("npix", [4, 8, 16, 100, 512, 2048])
+def test_flat_spectra_sizes(npix, two):
+    """Transforms with an odd and an even number of radix-2 stages, the smallest and a large
+    one, and a direct one, with bins narrower than a mode's spacing and wider.  FP64 FFTs
+    of different orders: 1e-11 of the largest value."""
+    import spectra
+    rng = np.random.default_rng(npix)
+    a = rng.standard_normal(npix * npix).astype(np.float32)
+    b = (a + rng.standard_normal(npix * npix)).astype(np.float32)
+    fov = float(np.float32(np.radians(10.0)))
+    # no mode on a bin's edge, where the last bit of ell decides
+    for ell_max, nbins in ((2 * np.pi / fov * npix * 0.4123457, 1000),
+                           (2 * np.pi / fov * npix * 0.3234561, 7)):
+        g = p2m.cl_flatsky(a, b if two else None, fov_rad=fov, ell_max=ell_max, nbins=nbins)
+        r = spectra.cl_flatsky(a, b if two else None, fov, ell_max, nbins)
+        assert np.array_equal(g["nmodes"], r["nmodes"])
+        for key in ("ell", "aa") + (("ab", "bb") if two else ()):
+            assert np.abs(g[key] - r[key]).max() <= 1e-11 * np.abs(r[key]).max()
