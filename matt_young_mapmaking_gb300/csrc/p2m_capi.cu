@@ -790,9 +790,8 @@ p2m_status sweep(p2m_ctx *ctx, cudaStream_t s) {
     /* fold the sparse low words into the maps and clear them */
     p2m_launch_fold_lo(P, W, s, ctx->nsm);
   } else {
-    /* the read-out reads the painted tiles; they are cleared after it for the next paint */
+    /* the read-out moves the painted tiles' sums to the maps and clears them */
     p2m_launch_read_tiles(P, W, ctx->swept ? 1 : 0, s, ctx->nsm);
-    p2m_launch_clear_tiles(P, W, s, ctx->nsm);
   }
   TE(PH_READOUT);
   CK(cudaGetLastError());

@@ -16,7 +16,7 @@
  *   scan + k_paint_full  the large halos' items, load-balanced over candidate pixels
  *   read-out   mixed precision: the maps hold the high words of a compensated sum and
  *              k_fold_lo adds the sparse low words; FP64 and fixed-point accumulation:
- *              k_read_tiles adds the painted tiles' sums, and k_clear_tiles clears them
+ *              k_read_tiles moves the painted tiles' sums to the maps
  */
 #ifndef P2M_INTERNAL_H
 #define P2M_INTERNAL_H
@@ -213,10 +213,9 @@ void p2m_launch_pair_table(float2 *dst, const float *ta, int pa, const float *tb
                            long long nent, cudaStream_t s, int nsm);
 void p2m_launch_paint_halos(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 void p2m_launch_paint_full(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
-/* read-out of the FP64 and fixed-point accumulators' flagged tiles into the maps; their clear */
+/* read-out and clear of the FP64 and fixed-point accumulators' flagged tiles */
 void p2m_launch_read_tiles(const PaintParams &P, const SweepBuffers &W, int add, cudaStream_t s,
                            int nsm);
-void p2m_launch_clear_tiles(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
 void p2m_launch_finalize_fs(const PaintParams &P, const void *acc, long long npix, float *out,
                             int map, double *sum, cudaStream_t s, int nsm);
 void p2m_launch_fold_lo(const PaintParams &P, const SweepBuffers &W, cudaStream_t s, int nsm);
