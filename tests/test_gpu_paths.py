@@ -5,6 +5,8 @@ import pytest
 
 import catalogs
 import matt_young_mapmaking_gb300 as p2m
+import oracle
+from test_gpu_parity import assert_maps_close
 
 pytestmark = pytest.mark.gpu
 
@@ -207,3 +209,25 @@ def test_flat_spectra_sizes(npix, two):
         assert np.array_equal(g["nmodes"], r["nmodes"])
         for key in ("ell", "aa") + (("ab", "bb") if two else ()):
             assert np.abs(g[key] - r[key]).max() <= 1e-11 * np.abs(r[key]).max()
+
+
+@pytest.mark.parametrize("npix_fs", [1, 33, 97])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fixed"])
+def test_flat_sky_readout_remainders(precision, npix_fs):
+    """Flat-sky maps whose pixel count is no multiple of a block's: each map against the
+    oracle, and the sum that the read-out adds up against the map's own (n FP64 additions
+    on either side: n 2^-52 of the sum of magnitudes)."""
+    rec = catalogs.cone(75, 20_000, (1.0, 0.0, 0.0), 8.0)
+    tab = catalogs.table(nu=0.0)
+    p = oracle.params(nside=0, npix_fs=npix_fs, maps=MAPS, nfloat=rec.shape[1], fov_deg=10.0)
+    rfs = oracle.paint(p, [oracle.Table(tab)], rec, record_sets=False)[1]
+    with p2m.Painter(nside=0, npix_fs=npix_fs, precision=precision, maps=MAPS, fov_deg=10.0,
+                     max_records=len(rec)) as pt:
+        pt.load_table(0, tab)
+        pt.paint_records(rec)
+        got = [pt.flatsky(m) for m in range(2)]
+        sums = pt.stats()["fs_sum"]
+    for m in range(2):
+        assert_maps_close(got[m], rfs[m], rel=1e-6, what="map %d" % m)
+        v = got[m].astype(np.float64)
+        assert abs(sums[m] - v.sum()) <= v.size * 2.0**-52 * np.abs(v).sum()
