@@ -722,21 +722,26 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   if (!ctx->unit_clean) ST(clear_call_counters(ctx, s));
   ctx->ctr_clean = ctx->unit_clean = false;
   PaintParams P = make_params(ctx, 7);
+  const bool keyed = ctx->tune.sort_halos && ctx->d_ring_hist;
+  const bool sorted = keyed && ctx->n_halos > unsorted_halos(ctx);
+  if (n > 0) CK(grow(&ctx->d_pix_off, &ctx->cap_pix_off, n));
+  if (sorted) CK(grow(&ctx->d_order, &ctx->cap_order, std::max(ctx->n_halos, 1LL)));
   TB(PH_GROUP);
   if (n > 0) {
-    /* candidate offsets of the large halos' items */
-    CK(grow(&ctx->d_pix_off, &ctx->cap_pix_off, n));
-    p2m_launch_scan_u32(ctx->d_counts, n, ctx->d_pix_off, &ctx->d_ctr->n_pix, ctx->d_scan_tmp, s);
+    /* candidate offsets of the large halos' items, on the side stream beside the sort */
+    CK(cudaEventRecord(ctx->ev_zero_start, s));
+    CK(cudaStreamWaitEvent(ctx->zstream, ctx->ev_zero_start, 0));
+    p2m_launch_scan_u32(ctx->d_counts, n, ctx->d_pix_off, &ctx->d_ctr->n_pix, ctx->d_scan_tmp,
+                        ctx->zstream);
   }
   SweepBuffers W = sweep_buffers(ctx);
-  if (ctx->tune.sort_halos && ctx->d_ring_hist && ctx->n_halos <= unsorted_halos(ctx)) {
+  if (keyed && !sorted) {
     ctx->hist_dirty = true;
-  } else if (ctx->tune.sort_halos && ctx->d_ring_hist) {
+  } else if (sorted) {
     /* counting sort of the halos by first ring (keys and counts came from the set-up):
        the halos painted at any one time then cover a narrow band of rings, a contiguous
        stretch of each map that the L2 holds */
     const long long nbins = 4LL * ctx->cfg.nside + 1;
-    CK(grow(&ctx->d_order, &ctx->cap_order, std::max(ctx->n_halos, 1LL)));
     p2m_launch_ring_scan(ctx->d_ring_hist, (int)nbins, ctx->d_ring_off, s);
     p2m_launch_ring_scatter(ctx->d_ring_key, ctx->n_halos, ctx->d_ring_off, ctx->d_order, s, ctx->nsm);
     W.order = ctx->d_order;
@@ -746,8 +751,6 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   if (n > 0) {
     /* the large halos' items are painted on the side stream, beside the fused kernel's
        uneven tail; the read-out waits for both */
-    CK(cudaEventRecord(ctx->ev_zero_start, s));
-    CK(cudaStreamWaitEvent(ctx->zstream, ctx->ev_zero_start, 0));
     tmark(ctx, PH_PAINT_BIG, 0, ctx->zstream);
     p2m_launch_paint_full(P, W, ctx->zstream, ctx->nsm);
     tmark(ctx, PH_PAINT_BIG, 1, ctx->zstream);
