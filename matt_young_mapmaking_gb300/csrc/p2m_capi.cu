@@ -1810,6 +1810,8 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   memcpy(b + 24, &th.mhmaxt, 4);
   memcpy(b + 28, &th.rmint, 4);
   memcpy(b + 32, &th.rmaxt, 4);
+  /* the image's fresh pages are faulted in while the kernel runs, not in the copy after it */
+  for (long long o = 4096; o < *nbytes; o += 4096) ((volatile char *)b)[o] = 0;
   CK(cudaMemcpyAsync(b + 36, d_tab, sizeof(float) * (size_t)th.nelem, cudaMemcpyDeviceToHost, sc.s));
   CK(cudaStreamSynchronize(sc.s));
   return P2M_OK;
