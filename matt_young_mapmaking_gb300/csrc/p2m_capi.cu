@@ -1783,7 +1783,7 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   /* scratch of this call, on a stream of its own */
   struct Scratch {
     cudaStream_t s = nullptr;
-    void *p[3] = {nullptr, nullptr, nullptr};
+    void *p[4] = {nullptr, nullptr, nullptr, nullptr};
     ~Scratch() {
       for (void *q : p) p2m_pool_free(q, s);
       if (s) cudaStreamDestroy(s);
@@ -1793,13 +1793,13 @@ p2m_status p2m_make_maptable(int32_t device, int32_t model, float nu, float alph
   CK(p2m_pool_alloc(&sc.p[0], sizeof(float) * P2M_NZTAB, sc.s));
   CK(p2m_pool_alloc(&sc.p[1], sizeof(float) * P2M_NZTAB, sc.s));
   CK(p2m_pool_alloc(&sc.p[2], sizeof(float) * (size_t)th.nelem, sc.s));
+  CK(p2m_pool_alloc(&sc.p[3], p2m_maptable_scratch(th), sc.s));
   float *d_rofz = (float *)sc.p[0], *d_zofr = (float *)sc.p[1], *d_tab = (float *)sc.p[2];
   CK(cudaMemcpyAsync(d_rofz, rofz.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice, sc.s));
   CK(cudaMemcpyAsync(d_zofr, zofr.data(), sizeof(float) * P2M_NZTAB, cudaMemcpyHostToDevice, sc.s));
   P.rofz = d_rofz;
   P.zofr = d_zofr;
-  p2m_launch_maptable(P, K, th, d_tab, sc.s);
-  CK(cudaGetLastError());
+  CK(p2m_launch_maptable(P, K, th, d_tab, sc.p[3], sc.s));
   char *b = (char *)image;
   memcpy(b + 0, &th.nchit, 4);
   memcpy(b + 4, &th.nmht, 4);

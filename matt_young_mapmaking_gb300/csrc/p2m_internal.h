@@ -250,7 +250,8 @@ struct TableConsts {
   int model;
   float neg_zero; /* -0: see mul2_sep */
 };
-void p2m_launch_maptable(const PaintParams &P, const TableConsts &K, const p2m_tabhdr &th,
-                         float *d_table, cudaStream_t s);
+size_t p2m_maptable_scratch(const p2m_tabhdr &th);
+cudaError_t p2m_launch_maptable(const PaintParams &P, const TableConsts &K, const p2m_tabhdr &th,
+                                float *d_table, void *scratch, cudaStream_t s);
 
 #endif

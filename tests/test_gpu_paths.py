@@ -231,3 +231,12 @@ def test_flat_sky_readout_remainders(precision, npix_fs):
         assert_maps_close(got[m], rfs[m], rel=1e-6, what="map %d" % m)
         v = got[m].astype(np.float64)
         assert abs(sums[m] - v.sum()) <= v.size * 2.0**-52 * np.abs(v).sum()
+
+
+@pytest.mark.parametrize("nchi,nm,nr", [(2, 2, 2), (3, 5, 127), (2, 3, 129), (300, 300, 2)])
+@pytest.mark.parametrize("model,nu", [(1, 0.0), (2, 353.0)])
+def test_table_sizes(model, nu, nchi, nm, nr):
+    """Tables below a warp, at the edges of a block of radii, and of more cells than one pass
+    takes: every entry is the reference's float sequence, so the image is the oracle's."""
+    assert p2m.make_maptable(model, nu, 0.0, nchit=nchi, nmht=nm, nrt=nr) == \
+        oracle.make_maptable(model, nu, 0.0, nchit=nchi, nmht=nm, nrt=nr)
