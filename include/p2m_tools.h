@@ -146,7 +146,8 @@ int32_t p2m_cl_flatsky(int32_t device, const float *map_a, const float *map_b, i
 /* Self-test of the single-precision math the kernels use (fn: 0 log, 1 exp, 2 pow,
    3 asin, 4 atan, 5 sin, 6 cos, 7 tan; 8 the fixed-point sum of P2M_PREC_FIXED:
    x and y each rounded to a multiple of 2^-56, added as integers and rounded back to
-   float) evaluated on the GPU over n device floats; d_y is read only for pow and 8.
+   float; 11 (x - 1) / (x + 1) for x in (1/sqrt 2, sqrt 2] and 12 x / y, as the table maker
+   divides) evaluated on the GPU over n device floats; d_y is read only for pow, 8 and 12.
    Synchronous.  Returns 0 or a CUDA error code. */
 int32_t p2m_fmath_eval_device(int32_t device, int32_t fn, const float *d_x, const float *d_y,
                               float *d_out, int64_t n);

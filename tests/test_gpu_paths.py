@@ -240,3 +240,28 @@ def test_table_sizes(model, nu, nchi, nm, nr):
     takes: every entry is the reference's float sequence, so the image is the oracle's."""
     assert p2m.make_maptable(model, nu, 0.0, nchit=nchi, nmht=nm, nrt=nr) == \
         oracle.make_maptable(model, nu, 0.0, nchit=nchi, nmht=nm, nrt=nr)
+
+
+@pytest.mark.parametrize("fn", [11, 12])
+def test_table_quotients_are_rounded(fn):
+    """The table maker's quotients are the IEEE ones: (m - 1) / (m + 1) at every mantissa that
+    the logarithm centres, and x / x_c over random distances and core radii and over the
+    mantissas next to powers of two."""
+    import torch
+    if fn == 11:
+        x = np.arange(0x3f3504f4, 0x3fb504f4, dtype=np.uint32).view(np.float32)
+        y, ref = x, (x - np.float32(1)) / (x + np.float32(1))
+    else:
+        rng = np.random.default_rng(76)
+        x = np.exp(rng.uniform(np.log(4e-3), np.log(8.0), 1 << 22)).astype(np.float32)
+        y = np.exp(rng.uniform(np.log(1e-2), np.log(10.0), 1 << 22)).astype(np.float32)
+        near = (np.array([1.0], np.float32).view(np.uint32) + np.arange(-1024, 1024)).astype(np.uint32)
+        y[: 1 << 20] = rng.choice(near, 1 << 20).view(np.float32)
+        x[1 << 19: 1 << 21] = rng.choice(near, 3 << 19).view(np.float32)
+        ref = x / y
+    dx, dy = torch.from_numpy(x.copy()).cuda(), torch.from_numpy(y.copy()).cuda()
+    out = torch.empty_like(dx)
+    assert p2m.load_library().p2m_fmath_eval_device(0, fn, dx.data_ptr(), dy.data_ptr(),
+                                                    out.data_ptr(), x.size) == 0
+    got = out.cpu().numpy()
+    assert np.array_equal(got, ref), "%d of %d differ" % ((got != ref).sum(), x.size)
