@@ -36,11 +36,11 @@ MASS = (1e12, 3e15)
 SEED = 2
 ZMAX = 6.0
 MAPS = ((0, 1), (0, 2))
-LAUNCHES_PER_STEP = 15
+LAUNCHES_PER_STEP = 10
 # DRAM bytes (read + write) per pixel update of k_paint_halos from an ncu capture of this
 # workload's launch (1e7 halos at Nside 4096, one pass: dram__bytes_read.sum +
-# dram__bytes_write.sum = 1.20 GB + 0.61 GB for 3.51e7 updates on each of two maps)
-PAINT_DRAM_BYTES_PER_UPDATE = 51.6
+# dram__bytes_write.sum = 1.40 GB + 0.59 GB for 3.51e7 updates on each of two maps)
+PAINT_DRAM_BYTES_PER_UPDATE = 56.6
 # L2 atomic throughput of this GB300 (sectors/s): ncu lts__t_sectors_srcunit_tex_op_atom
 # of the same capture, 26.7 sectors/ns at 7.06 % of peak sustained
 L2_ATOMIC_SECTORS_PER_S = 3.79e11
@@ -804,10 +804,9 @@ def run_ours(args):
                    "sequential": {"value": total_halos / (e2e_seq_ms * 1e-3),
                                   "ms_per_step": e2e_seq_ms},
                    "maps_vs_resident_max_rel": e2e_check}}
-    # per step: the fused cut and set-up, the item kernel of the large halos, their
-    # candidate counts and 3-kernel scan, the painting order's 3-kernel scan and scatter,
-    # the fused paint, the large-halo paint, the fold of the low words, and the two
-    # counter read-outs (memsets are not kernels)
+    # per step: the fused cut and set-up, the item kernel of the large halos, their 3-kernel
+    # scan, the painting order's one-block scan and scatter, the large-halo paint, the fused
+    # paint, and the fold of the low words (memsets are not kernels)
     out["gpu_launches"] = LAUNCHES_PER_STEP * args.steps
 
     plain_maps = None

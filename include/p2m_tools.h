@@ -30,8 +30,9 @@ void p2m_philox4x32(const uint32_t c[4], const uint32_t k[2], uint32_t out[4]);
 /* Device time (ms) of each phase of the last paint call and of the last map read-out,
    for a context created with P2M_FLAG_TIMING: [0] cut with the per-halo set-up of
    catalogue records (one kernel), [1] set-up of p2m_project_halo batches, [2] unused
-   (0: the large halos reserve their item ranges during the set-up), [3] their ring spans, [4] flat sky, [5] their candidate
-   offsets, [6] HEALPix paint (both painting kernels, which run concurrently), [7] the
+   (0: the large halos reserve their item ranges during the set-up), [3] their ring spans,
+   [4] flat sky, [5] the painting order (their candidate offsets are scanned beside it),
+   [6] HEALPix paint (both painting kernels, which run concurrently), [7] the
    large halos' painting kernel alone, [8] read-out.  Diagnostics only (the reference prints no
    timings). */
 struct p2m_ctx;
@@ -65,18 +66,21 @@ typedef struct p2m_tuning {
   int32_t halos_grid; /* 128-thread blocks per SM of the fused enumerate-and-paint kernel
                          (8 fit at once), 1..16; 8 */
   int32_t full_grid;  /* blocks per SM of the stored-item kernel, 1..32; 8 */
-  int32_t full_chunk; /* candidates per warp chunk of the stored-item kernel, 32..65536; 1024 */
+  int32_t full_chunk; /* candidates per warp chunk of the stored-item kernel, at most (fewer,
+                         down to 256, where that would leave warps without work), 32..65536;
+                         1024 */
   int32_t stream_chunk; /* host records per chunk of the streamed ingest of p2m_paint_records
                            (copy of chunk k+1 overlapped with chunk k), 65536..2^26; 2^22 */
   int32_t stream_paint; /* 1: whenever a full chunk's worth of records (this call's or
                            earlier calls') awaits painting, paint it before the next chunk is
                            ingested, so that the copies overlap the painting too; 0: paint
                            at the read-out; 1 */
-  int32_t halo_batch; /* halos per warp batch of the fused kernel, 1..32; 16 */
+  int32_t halo_batch; /* halos per warp batch of the fused kernel, at most (fewer where that
+                         would leave warps without a batch), 1..32; 16 */
   int32_t sort_halos; /* 1: paint the halos in order of their first ring (a counting sort:
                          the set-up counts the keys, the paint scans and scatters them), so
-                         that the halos in flight cover a narrow band of the maps; 0: in
-                         catalogue order; 1 */
+                         that the halos in flight cover a narrow band of the maps; not done
+                         where all of them are in flight at once); 0: in catalogue order; 1 */
   int32_t halos_threads; /* threads per block of the fused kernel, 128 or 256 (halos_grid
                             blocks of them per SM); 128 */
   /* No table-tile field: the profile tables are read through the read-only cache
@@ -118,7 +122,7 @@ int32_t p2m_write_flatsky(const char *path, const float *map, int32_t npix, floa
 int32_t p2m_write_healpix_fits(const char *path, const float *map, int32_t nside);
 
 /* Angular power spectra of painted maps, for the precision report (validation only;
-   host maps in, spectra out, synchronous, device memory allocated for the call).
+   host maps in, spectra out, synchronous, device memory from a pool that keeps 256 MB).
 
    p2m_cl_healpix: the spectra of RING-ordered HEALPix maps up to lmax (<= 4 nside and
    <= P2M_CL_LMAX_MAX), by the pixel-area quadrature of the HEALPix library that the

@@ -728,7 +728,9 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   if (sorted) CK(grow(&ctx->d_order, &ctx->cap_order, std::max(ctx->n_halos, 1LL)));
   TB(PH_GROUP);
   if (n > 0) {
-    /* candidate offsets of the large halos' items, on the side stream beside the sort */
+    /* candidate offsets of the large halos' items, on the side stream, whose kernel alone reads
+       them, beside the sort: y of 1e6 halos at Nside 2048, 152 us a pass with the scan before
+       the sort, 141 us here */
     CK(cudaEventRecord(ctx->ev_zero_start, s));
     CK(cudaStreamWaitEvent(ctx->zstream, ctx->ev_zero_start, 0));
     p2m_launch_scan_u32(ctx->d_counts, n, ctx->d_pix_off, &ctx->d_ctr->n_pix, ctx->d_scan_tmp,

@@ -13,7 +13,8 @@
  * Sweep:
  *   k_paint_halos  the other halos, enumeration fused with painting: a warp builds the
  *              ring spans of a batch of halos in registers and paints their candidates
- *   scan + k_paint_full  the large halos' items, load-balanced over candidate pixels
+ *   scan + k_paint_full  the large halos' items, load-balanced over candidate pixels, on the
+ *              side stream
  *   read-out   mixed precision: the maps hold the high words of a compensated sum and
  *              k_fold_lo adds the sparse low words; FP64 and fixed-point accumulation:
  *              k_read_tiles moves the painted tiles' sums to the maps

@@ -25,7 +25,7 @@
  *             each ring pair (north and mirror) is split into its four interleaved quarters
  *             of n pixels, for the sums S = north + south and the differences
  *             D = north - south, with both maps in one complex sequence (a + i b).
- *             k_quarter_fft transforms the quarters in shared memory: radix 2 when n is a
+ *             k_quarter_fft transforms the quarters in shared memory: radix 4 when n is a
  *             power of two (all belt rings), Bluestein's chirp convolution otherwise
  *             (k_chirp prepares each cap ring's chirp transform), in two halves where its
  *             length is over QF_MAX_CONV.  k_ring_combine joins the quarters for every m, separates the
@@ -42,7 +42,7 @@
  *   C(ell) = (fov^2 / npix^4) |FFT(map)(k)|^2, averaged over the modes of a bin
  *
  * k = 0 is left out, and so is the Nyquist line.  Both maps go through one complex FFT
- * (a + i b).  The rows are transformed by a radix-2 FFT in shared memory when npix is
+ * (a + i b).  The rows are transformed by a radix-4 FFT in shared memory when npix is
  * a power of two up to 8192, or by a direct DFT for other npix up to 2048.  The columns
  * are transformed the same way after a transpose.
  */
