@@ -800,6 +800,19 @@ struct Stream {
     }                                                              \
   } while (0)
 
+/* allows a kernel the most dynamic shared memory that any call asks of it.  The limit belongs to
+   the kernel, not to the launch: set to what one call needs, it could be lowered by another
+   thread's smaller call before the launch, which would then be refused. */
+template <class K>
+cudaError_t allow_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+constexpr size_t QF_SMEM = sizeof(double2) * QF_MAX_CONV;
+constexpr size_t FFT_SMEM = sizeof(double2) * FFT_MAX_POW2;
+constexpr size_t alm_smem(int group) {
+  return sizeof(double) * ((size_t)group * 8 + 2 * ALM_LC + (size_t)ALM_WARPS * ALM_LC * 4);
+}
+
 bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 int ilog2(int n) {
   int l = 0;
@@ -873,8 +886,8 @@ int32_t p2m_cl_healpix(int32_t device, const float *map_a, const float *map_b, i
   k_twiddles<<<(twlen / 2 + 256) / 256, 256, 0, st.s>>>(d_tw, twlen);
   SP_CK(cudaGetLastError());
   const size_t fsmem = sizeof(double2) * (size_t)longest;
-  SP_CK(cudaFuncSetAttribute(k_chirp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
-  SP_CK(cudaFuncSetAttribute(k_quarter_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+  SP_CK(allow_smem(k_chirp, QF_SMEM));
+  SP_CK(allow_smem(k_quarter_fft, QF_SMEM));
   if (nside > 1) {
     k_chirp<<<nside - 1, QF_THREADS, fsmem, st.s>>>(d_off, d_tw, twlen, d_chirp);
     SP_CK(cudaGetLastError());
@@ -887,13 +900,12 @@ int32_t p2m_cl_healpix(int32_t device, const float *map_a, const float *map_b, i
   SP_CK(cudaGetLastError());
   SP_CK(cudaMemsetAsync(d_alm, 0, sizeof(double) * 4 * nalm, st.s));
   const int group = std::min(ALM_GROUP, (nrings + ALM_THREADS - 1) / ALM_THREADS * ALM_THREADS);
-  const size_t smem = sizeof(double) * ((size_t)group * 8 + 2 * ALM_LC +
-                                        (size_t)ALM_WARPS * ALM_LC * 4);
+  const size_t smem = alm_smem(group);
   if (map_b) {
-    SP_CK(cudaFuncSetAttribute(k_alm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SP_CK(allow_smem(k_alm<true>, alm_smem(ALM_GROUP)));
     k_alm<true><<<lmax + 1, ALM_THREADS, smem, st.s>>>(d_ph, d_mfac, nside, lmax, group, d_alm);
   } else {
-    SP_CK(cudaFuncSetAttribute(k_alm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SP_CK(allow_smem(k_alm<false>, alm_smem(ALM_GROUP)));
     k_alm<false><<<lmax + 1, ALM_THREADS, smem, st.s>>>(d_ph, d_mfac, nside, lmax, group, d_alm);
   }
   SP_CK(cudaGetLastError());
@@ -946,8 +958,8 @@ int32_t p2m_cl_flatsky(int32_t device, const float *map_a, const float *map_b, i
   if (pow2) {
     const int logn = ilog2(npix);
     const size_t smem = sizeof(double2) * (size_t)npix;
-    SP_CK(cudaFuncSetAttribute(k_fft_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SP_CK(cudaFuncSetAttribute(k_fft_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SP_CK(allow_smem(k_fft_rows<1>, FFT_SMEM));
+    SP_CK(allow_smem(k_fft_rows<0>, FFT_SMEM));
     k_twiddles<<<(npix / 2 + 255) / 256, 256, 0, st.s>>>(tw, npix);
     k_fft_rows<1><<<npix, FFT_THREADS, smem, st.s>>>(z, d_a, d_b, npix, logn, tw);
     k_transpose<<<tg, tb, 0, st.s>>>(z, z2, npix);
