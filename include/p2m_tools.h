@@ -122,7 +122,8 @@ int32_t p2m_write_flatsky(const char *path, const float *map, int32_t npix, floa
 int32_t p2m_write_healpix_fits(const char *path, const float *map, int32_t nside);
 
 /* Angular power spectra of painted maps, for the precision report (validation only;
-   host maps in, spectra out, synchronous, device memory from a pool that keeps 256 MB).
+   host maps in, spectra out, synchronous, device memory from a pool that keeps 256 MB; usable
+   after a cudaDeviceReset).
 
    p2m_cl_healpix: the spectra of RING-ordered HEALPix maps up to lmax (<= 4 nside and
    <= P2M_CL_LMAX_MAX), by the pixel-area quadrature of the HEALPix library that the
@@ -130,7 +131,9 @@ int32_t p2m_write_healpix_fits(const char *path, const float *map, int32_t nside
    (src/modules/External/alm_map_dd_inc.F90:2978-3224, ring_analysis and the lambda_lm
    recursion of alm_tools.F90:394-650, 1022-1097), then alm2cl (alm_map_dd_inc.F90:5347-5423).
    cl_aa[l], and with map_b, cl_ab[l] = sum_m Re a_lm conj(b_lm) / (2l+1) and cl_bb[l],
-   for l = 0 .. lmax.  map_b may be NULL (cl_ab and cl_bb are then not written).
+   for l = 0 .. lmax.  map_b may be NULL (cl_ab and cl_bb are then not written).  Device memory:
+   about 192 nside^2 bytes for the rings' transforms (13 GB at Nside 8192), up to 120 nside^2 for
+   the maps and the chirps, 128 nside (lmax + 1) for the phases and 16 (lmax + 1)^2 for the a_lm.
 
    p2m_cl_flatsky: binned periodogram of npix x npix flat-sky maps over fov_rad x fov_rad
    (the layout of p2m_get_flatsky): nbins (<= P2M_CL_MAXBINS) linear bins of ell = 2 pi |k| / fov in

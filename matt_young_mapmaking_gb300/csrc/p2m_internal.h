@@ -240,7 +240,7 @@ void p2m_launch_ring_scatter(const int *keys, long long n, long long *off, int *
 void p2m_launch_ring_unhist(const int *keys, long long n, unsigned int *hist, cudaStream_t s,
                             int nsm);
 /* Stream-ordered device memory for the calls that need scratch for their own duration only (the
-   spectra, the table maker), from a pool of the current device that keeps up to 256 MB between
+   spectra, the table maker), from a pool of the current context that keeps up to 256 MB between
    calls (any thread's and stream's) and returns the rest when a stream is waited for: making
    and dropping such buffers took half of a 1024^2 flat-sky call.  Free on the same stream. */
 cudaError_t p2m_pool_alloc(void **out, size_t bytes, cudaStream_t s);

@@ -46,6 +46,7 @@
  * a power of two up to 8192, or by a direct DFT for other npix up to 2048.  The columns
  * are transformed the same way after a transpose.
  */
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,22 +62,51 @@
 
 namespace {
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pools[64] = {};
+struct ContextPool {
+  unsigned long long context;
+  cudaMemPool_t pool;
+};
+std::vector<ContextPool> g_pools;
+
+/* the driver's id of the current context, which no other context of this process ever has */
+cudaError_t context_id(unsigned long long *id) {
+  struct Entry {
+    void *fn = nullptr;
+    Entry(const char *name, unsigned version) {
+      cudaDriverEntryPointQueryResult found;
+      if (cudaGetDriverEntryPointByVersion(name, &fn, version, cudaEnableDefault, &found) !=
+              cudaSuccess ||
+          found != cudaDriverEntryPointSuccess)
+        fn = nullptr;
+    }
+  };
+  static const Entry get_current("cuCtxGetCurrent", 4000), get_id("cuCtxGetId", 12000);
+  if (!get_current.fn || !get_id.fn) return cudaErrorNotSupported;
+  CUcontext ctx = nullptr;
+  if (((CUresult (*)(CUcontext *))get_current.fn)(&ctx) != CUDA_SUCCESS || !ctx ||
+      ((CUresult (*)(CUcontext, unsigned long long *))get_id.fn)(ctx, id) != CUDA_SUCCESS)
+    return cudaErrorInvalidDevice;
+  return cudaSuccess;
+}
 }  // namespace
 
+/* A pool belongs to the context that it was made in: after a cudaDeviceReset the next call makes
+   another (what is kept of the old one is its entry in the list). */
 cudaError_t p2m_pool_alloc(void **out, size_t bytes, cudaStream_t s) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  unsigned long long context = 0;
+  cudaError_t e = context_id(&context);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  cudaMemPool_t pool;
+  cudaMemPool_t pool = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (!g_pools[dev]) {
+    for (const ContextPool &c : g_pools)
+      if (c.context == context) pool = c.pool;
+    if (!pool) {
       cudaMemPoolProps props = {};
       props.allocType = cudaMemAllocationTypePinned;
       props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
+      e = cudaGetDevice(&props.location.id);
+      if (e != cudaSuccess) return e;
       cudaMemPool_t made;
       e = cudaMemPoolCreate(&made, &props);
       if (e != cudaSuccess) return e;
@@ -86,9 +116,9 @@ cudaError_t p2m_pool_alloc(void **out, size_t bytes, cudaStream_t s) {
         cudaMemPoolDestroy(made);
         return e;
       }
-      g_pools[dev] = made;
+      g_pools.push_back({context, made});
+      pool = made;
     }
-    pool = g_pools[dev];
   }
   return cudaMallocFromPoolAsync(out, bytes ? bytes : 1, pool, s);
 }
