@@ -66,7 +66,8 @@ struct p2m_ctx {
   long long cap_order = 0, cap_ring_key = 0;
   unsigned int *d_ring_hist = nullptr;
   long long *d_ring_off = nullptr;
-  bool hist_dirty = false; /* it holds counts of halos that were painted without a sort */
+  bool hist_dirty = false; /* it holds counts of other halos than those that await painting:
+                              painted without a sort, or of an ingest that failed */
   /* outputs: hp_npix counts every cone's pixels (ncones * cone_npix) */
   long long hp_npix = 0, fs_npix = 0;
   long long cone_npix = 0;
@@ -171,7 +172,10 @@ cudaError_t grow(T **p, long long *cap, long long need, long long keep = 0, cuda
   long long n = std::max(need + need / 4, (long long)1024);
   T *q = nullptr;
   cudaError_t e = cudaMalloc((void **)&q, sizeof(T) * (size_t)n);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) {
+    cudaGetLastError(); /* reported by this call, not by the next launch */
+    return e;
+  }
   if (*p && keep > 0) {
     e = cudaMemcpyAsync(q, *p, sizeof(T) * (size_t)keep, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -421,15 +425,7 @@ p2m_status wait_counters(p2m_ctx *ctx, cudaStream_t s) {
 p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, bool handed, cudaStream_t s) {
   IngestBuffers B = ingest_buffers(ctx, nullptr);
   /* the large halos reserved their item ranges (d_ioff, n_items) during the set-up */
-  const p2m_status err = handed ? wait_counters(ctx, s) : read_counters(ctx, s);
-  if (err) {
-    /* the call is discarded: its halos, stored past n_halos, are overwritten by the next
-       call, and they leave the first-ring counts that the next sort scans */
-    if (ctx->tune.sort_halos && ctx->d_ring_hist && ctx->h_ctr->n_surv > 0)
-      p2m_launch_ring_unhist(ctx->d_ring_key + ctx->n_halos, (long long)ctx->h_ctr->n_surv,
-                             ctx->d_ring_hist, s, ctx->nsm);
-    return err;
-  }
+  ST(handed ? wait_counters(ctx, s) : read_counters(ctx, s));
   long long n_halo = (long long)ctx->h_ctr->n_surv;
   long long n_items = P.nside > 0 ? (long long)ctx->h_ctr->n_items : 0;
   long long n_fs = (long long)ctx->h_ctr->n_fs_rows;
@@ -452,6 +448,7 @@ p2m_status ingest_tail(p2m_ctx *ctx, const PaintParams &P, bool handed, cudaStre
     }
   }
   CK(cudaGetLastError());
+  ctx->hist_dirty = false;
   ctx->n_halos += n_halo;
   ctx->n_items += n_items;
   if (n_halo > 0) ctx->dirty = true;
@@ -511,6 +508,19 @@ p2m_status wait_zero(p2m_ctx *ctx, cudaStream_t s) {
   return P2M_OK;
 }
 
+/* makes the first-ring counts those of the halos that await painting.  A sort over counts of
+   others would send halos' places past the end of their order. */
+p2m_status restore_hist(p2m_ctx *ctx, cudaStream_t s) {
+  if (!ctx->hist_dirty) return P2M_OK;
+  CK(cudaMemsetAsync(ctx->d_ring_hist, 0, ring_hist_bytes(ctx), s));
+  if (ctx->tune.sort_halos && ctx->n_halos > 0) { /* they have keys: see begin_call */
+    p2m_launch_ring_hist(ctx->d_ring_key, ctx->n_halos, ctx->d_ring_hist, s, ctx->nsm);
+    CK(cudaGetLastError());
+  }
+  ctx->hist_dirty = false;
+  return P2M_OK;
+}
+
 p2m_status begin_call(p2m_ctx *ctx, long long n, cudaStream_t s) {
   ST(zero_outputs(ctx, s));
   CK(grow(&ctx->d_nring, &ctx->cap_nring, std::max(n, 1LL)));
@@ -525,13 +535,13 @@ p2m_status begin_call(p2m_ctx *ctx, long long n, cudaStream_t s) {
       CK(cudaMalloc((void **)&ctx->d_ring_off, sizeof(long long) * (size_t)nbins));
     }
   }
-  if (ctx->hist_dirty) {
-    CK(cudaMemsetAsync(ctx->d_ring_hist, 0, ring_hist_bytes(ctx), s));
-    ctx->hist_dirty = false;
-  }
+  ST(restore_hist(ctx, s));
   for (int k = 0; k < P2M_NPHASE; k++) ctx->tev_used[k] = false;
   if (!ctx->ctr_clean) ST(clear_call_counters(ctx, s));
   ctx->ctr_clean = false;
+  /* the set-up counts this call's halos: should the call fail from here on, it is discarded, its
+     halos, stored past n_halos, are overwritten by the next call, and the counts are made anew */
+  ctx->hist_dirty = ctx->tune.sort_halos && ctx->d_ring_hist;
   return P2M_OK;
 }
 
@@ -670,8 +680,10 @@ p2m_status ingest_device(p2m_ctx *ctx, const float *d_rec, long long nrec, int n
   TB(PH_CUT);
   p2m_launch_cut_setup(P, B, nrec, s, ctx->nsm);
   TE(PH_CUT);
-  CK(cudaGetLastError());
-  p2m_status st = ingest_tail(ctx, P, true, s);
+  const cudaError_t e = cudaGetLastError();
+  const p2m_status st = e == cudaSuccess
+                            ? ingest_tail(ctx, P, true, s)
+                            : fail(ctx, P2M_ERR_CUDA, std::string("cut: ") + cudaGetErrorString(e));
   join_out(ctx, s);
   if (st) return st;
   ctx->rec_count += nrec;
@@ -744,6 +756,7 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
        the halos painted at any one time then cover a narrow band of rings, a contiguous
        stretch of each map that the L2 holds */
     const long long nbins = 4LL * ctx->cfg.nside + 1;
+    ST(restore_hist(ctx, s));
     p2m_launch_ring_scan(ctx->d_ring_hist, (int)nbins, ctx->d_ring_off, s);
     p2m_launch_ring_scatter(ctx->d_ring_key, ctx->n_halos, ctx->d_ring_off, ctx->d_order, s, ctx->nsm);
     W.order = ctx->d_order;

@@ -236,9 +236,9 @@ void p2m_launch_copy_counters(const DevCounters *d, DevCounters *h_mapped, cudaS
    consumed */
 void p2m_launch_ring_scatter(const int *keys, long long n, long long *off, int *order,
                              cudaStream_t s, int nsm);
-/* takes halos [0, n) of a discarded ingest back out of the first-ring counts */
-void p2m_launch_ring_unhist(const int *keys, long long n, unsigned int *hist, cudaStream_t s,
-                            int nsm);
+/* counts the halos [0, n) by first ring, as the set-up does */
+void p2m_launch_ring_hist(const int *keys, long long n, unsigned int *hist, cudaStream_t s,
+                          int nsm);
 /* Stream-ordered device memory for the calls that need scratch for their own duration only (the
    spectra, the table maker), from a pool of the current context that keeps up to 256 MB between
    calls (any thread's and stream's) and returns the rest when a stream is waited for: making
