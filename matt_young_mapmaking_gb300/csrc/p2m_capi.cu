@@ -406,8 +406,14 @@ p2m_status read_counters(p2m_ctx *ctx, cudaStream_t s) {
 
 /* waits for the counters that k_cut_setup, queued on s, hands over with sequence number
    ctx->seq.  The host polls the number: a wait for the stream costs several us more.  Should
-   the stream end without it, its error (or the missing number) is reported. */
+   the stream end without it, its error (or the missing number) is reported.  Polling takes a
+   core, as the CUDA runtime's own waits do by default; where the program has asked the device
+   to yield or block instead (cudaSetDeviceFlags), the stream is waited for. */
 p2m_status wait_counters(p2m_ctx *ctx, cudaStream_t s) {
+  unsigned int flags = 0;
+  CK(cudaGetDeviceFlags(&flags));
+  if (flags & (cudaDeviceScheduleYield | cudaDeviceScheduleBlockingSync))
+    CK(cudaStreamSynchronize(s));
   for (unsigned spin = 1; *ctx->h_seq != ctx->seq; spin++) {
     if (spin & 0xfff) continue;
     const cudaError_t e = cudaStreamQuery(s);
