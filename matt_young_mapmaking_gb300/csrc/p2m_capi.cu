@@ -227,9 +227,12 @@ size_t ring_hist_bytes(const p2m_ctx *ctx) {
   return sizeof(unsigned int) * (size_t)(4LL * ctx->cfg.nside + 1);
 }
 
-/* Up to this many halos are painted at once (a batch for every resident warp of the fused
-   kernel): they are not sorted, as an order would not change which are in flight.  Their
-   sort, of 2e4 records at Nside 256, took 22 us of a pass of 57. */
+/* Up to this many halos are painted without a sort: a batch for each warp of 1024 threads an SM,
+   which builds of the fused kernel with so many resident threads paint all at once, so that an
+   order would not change which are in flight.  Their sort, of 2e4 records at Nside 256, took 22 us
+   of a pass of 57.  The compensated build for more than two maps has 768 resident threads and
+   paints the last quarter later, but is the faster unsorted too: six maps of 60,000 and 77,000
+   halos at Nside 4096 take 1145 and 1230 us a pass, sorted 1224 and 1327. */
 long long unsorted_halos(const p2m_ctx *ctx) {
   return (long long)ctx->nsm * std::min(ctx->tune.halos_grid * ctx->tune.halos_threads, 1024) /
          32 * ctx->tune.halo_batch;
@@ -744,7 +747,6 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
   const bool sorted = keyed && ctx->n_halos > unsorted_halos(ctx);
   if (n > 0) CK(grow(&ctx->d_pix_off, &ctx->cap_pix_off, n));
   if (sorted) CK(grow(&ctx->d_order, &ctx->cap_order, std::max(ctx->n_halos, 1LL)));
-  TB(PH_GROUP);
   if (n > 0) {
     /* candidate offsets of the large halos' items, on the side stream, whose kernel alone reads
        them, beside the sort: y of 1e6 halos at Nside 2048, 152 us a pass with the scan before
@@ -763,11 +765,12 @@ p2m_status paint_pending(p2m_ctx *ctx, cudaStream_t s) {
        stretch of each map that the L2 holds */
     const long long nbins = 4LL * ctx->cfg.nside + 1;
     ST(restore_hist(ctx, s));
+    TB(PH_GROUP);
     p2m_launch_ring_scan(ctx->d_ring_hist, (int)nbins, ctx->d_ring_off, s);
     p2m_launch_ring_scatter(ctx->d_ring_key, ctx->n_halos, ctx->d_ring_off, ctx->d_order, s, ctx->nsm);
+    TE(PH_GROUP);
     W.order = ctx->d_order;
   }
-  TE(PH_GROUP);
   TB(PH_PAINT); /* the paint phase spans both painting kernels */
   if (n > 0) {
     /* the large halos' items are painted on the side stream, beside the fused kernel's
