@@ -12,6 +12,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 #include <vector>
@@ -299,7 +300,8 @@ PaintParams make_params(const p2m_ctx *ctx, int nfloat) {
     const float dr = 1e-5f;
     P.r_out = ctx->th.rmaxt * (1.0f + dr);
     P.r_in = ctx->th.rmaxt * (1.0f - dr);
-    P.r_min_in = ctx->th.rmint * (1.0f + dr);
+    /* the fast decision's logarithm is for normal floats */
+    P.r_min_in = std::max(ctx->th.rmint * (1.0f + dr), std::numeric_limits<float>::min());
     P.r_min_out = ctx->th.rmint * (1.0f - dr);
     P.row_m = ctx->th.nrt;
     P.row_c = ctx->th.nrt * ctx->th.nmht;

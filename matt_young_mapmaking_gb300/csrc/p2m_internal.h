@@ -113,8 +113,9 @@ struct PaintParams {
   float fr_c;
   float band_u;  /* half-width of the r-index recheck band (cell units) */
   float inv_drt; /* 1 / drt of the table */
-  float r_out, r_in, r_min_in, r_min_out; /* rmaxt (1 +- 1e-5) and rmint (1 -+ 1e-5): radii
-                    between a pair are left to the exact path */
+  float r_out, r_in, r_min_in, r_min_out; /* rmaxt (1 +- 1e-5) and rmint (1 +- 1e-5), r_min_in
+                    at least the smallest normal float: radii between a pair are left to the
+                    exact path */
   float neg_zero;   /* -0: see mul2_sep */
   int row_m, row_c; /* float2 entries from a table row to the next mass and the next chi */
   int big_rings; /* halos spanning more rings are painted from stored items */

@@ -265,3 +265,36 @@ def test_table_quotients_are_rounded(fn):
                                                     out.data_ptr(), x.size) == 0
     got = out.cpu().numpy()
     assert np.array_equal(got, ref), "%d of %d differ" % ((got != ref).sum(), x.size)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fixed", "fp64"])
+def test_subnormal_radii_equal_the_exact_path(precision, monkeypatch):
+    """A table whose first radii are subnormal floats: the fast logarithm is for normal ones, so
+    such candidates take the exact path, and the maps are those of every candidate's exact path.
+    The sums' order is the only difference: to one float ulp."""
+    nchi, nm, nr = 3, 3, 60
+    header = np.array([nchi, nm, nr], np.int32).tobytes() + np.array(
+        [1e-37, 1e-35, 1e13, 1e16, 1e-41, 2e-37], np.float32).tobytes()
+    rng = np.random.default_rng(5)
+    image = header + rng.uniform(0.5, 1.5, 2 * nchi * nm * nr).astype(np.float32).tobytes()
+    z = np.linspace(0.0, 6.0, 10000).astype(np.float32)
+    rofz = np.linspace(0.0, 6e-36, 10000).astype(np.float32)
+
+    def maps():
+        with p2m.Painter(nside=512, precision=precision, maps=MAPS, zmax=6.0) as pt:
+            pt.set_cosmology_tables(rofz, z, 6.0, 6000.0)
+            pt.load_table(0, image)
+            for k in range(40):
+                v = np.random.default_rng(k).standard_normal(3)
+                x, y, w = (1000.0 * v / np.linalg.norm(v)).tolist()
+                pt.project_halo(x, y, w, 8.0, 1000.0, 1e14, 1.0, 1.0, 1 + (k & 1))
+            out = [pt.healpix(m) for m in range(2)]
+            return out, pt.stats()["hp_updates"]
+
+    fast, n1 = maps()
+    monkeypatch.setenv("P2M_BAND_U", "2")
+    exact, n2 = maps()
+    assert n1 == n2 > 10_000
+    for a, b in zip(fast, exact):
+        assert a.any()
+        assert np.all(np.abs(a - b) <= np.spacing(np.maximum(np.abs(a), np.abs(b))))
