@@ -218,7 +218,9 @@ p2m_status p2m_get_healpix_device(p2m_ctx *ctx, int32_t map, float *d_out, void 
    the storage of HEALPix map `map`
    (the reference's hpmap allocation, pks2map.f90:113): read-outs then write it in place
    and p2m_get_healpix_device with the same pointer copies nothing.  Call right after
-   p2m_create or p2m_reset_maps; NULL restores the context's own buffer. */
+   p2m_create or p2m_reset_maps; NULL restores the context's own buffer.  The first paint call
+   clears the buffer, in every precision, and read-outs then write the painted pixels: from
+   that call to the next p2m_reset_maps nothing else may write it. */
 p2m_status p2m_bind_healpix_device(p2m_ctx *ctx, int32_t map, float *d_out);
 
 /* Statistics of one map as a read-out delivers it (pks2map.f90:321-334): the moments

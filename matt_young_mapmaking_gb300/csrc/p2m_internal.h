@@ -121,7 +121,7 @@ struct PaintParams {
   int big_rings; /* halos spanning more rings are painted from stored items */
   const float *tables[P2M_MAXTABLES];
   /* maps 2q and 2q + 1 as one table of float2 entries (.x map 2q, .y map 2q + 1) at the
-     tables' float2 index cb / 2 + ir - 1: the table itself where the pair is profiles 1
+     float2 index cb + ir - 1: the table itself where the pair is profiles 1
      and 2 of one table (or a lone last map of profile 1), else a gathered copy */
   const float2 *pair_tab[P2M_MAXMAPS / 2];
   const float *rofz, *zofr;

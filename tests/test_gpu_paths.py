@@ -298,3 +298,13 @@ def test_subnormal_radii_equal_the_exact_path(precision, monkeypatch):
     for a, b in zip(fast, exact):
         assert a.any()
         assert np.all(np.abs(a - b) <= np.spacing(np.maximum(np.abs(a), np.abs(b))))
+
+
+@pytest.mark.parametrize("nchi,nm,nr", [(2, 2, 200), (3, 7, 129)])
+@pytest.mark.parametrize("model,nu,alpha", [(3, 0.0, 0.0), (3, 217.0, 0.02), (2, 0.0, 0.0)])
+def test_table_models_at_their_largest_exponents(model, nu, alpha, nchi, nm, nr):
+    """Model 3, and model 2 without a frequency, with the smallest and the largest mass at the
+    nearest and the farthest distance, where the profiles' exponents are largest: every entry is
+    the reference's float sequence, so the image is the oracle's."""
+    assert p2m.make_maptable(model, nu, alpha, nchit=nchi, nmht=nm, nrt=nr) == \
+        oracle.make_maptable(model, nu, alpha, nchit=nchi, nmht=nm, nrt=nr)
