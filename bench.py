@@ -40,7 +40,7 @@ LAUNCHES_PER_STEP = 10
 # DRAM bytes (read + write) per pixel update of k_paint_halos from an ncu capture of this
 # workload's launch (1e7 halos at Nside 4096, one pass: dram__bytes_read.sum +
 # dram__bytes_write.sum = 1.40 GB + 0.59 GB for 3.51e7 updates on each of two maps)
-PAINT_DRAM_BYTES_PER_UPDATE = 56.6
+PAINT_DRAM_BYTES_PER_UPDATE = 56.8
 # L2 atomic throughput of this GB300 (sectors/s): ncu lts__t_sectors_srcunit_tex_op_atom
 # of the same capture, 26.7 sectors/ns at 7.06 % of peak sustained
 L2_ATOMIC_SECTORS_PER_S = 3.79e11
